@@ -128,6 +128,8 @@ struct sphgpu_scene {
     // priority, so the records the sweeps gather stay resident (measured at
     // 1 M: density sweeps A/B 135/74 -> 129/72 us; records evict-last: no gain)
     int l2pol = 1;
+    // the list build (SolverConst::build): -1 by size, else 0 or 1 (debug knob "build")
+    int build = -1;
     int fuse_div = 1;  // DFSPH: the list build performs the divergence loop's first sweep A
     int fuse_ws = 1;   // warm start: features and inference in one kernel
     // set while a step that is not its call's last is enqueued: the step's
@@ -250,6 +252,13 @@ GridGeom make_grid(const SphParams& P) {
     return g;
 }
 
+// Scenes of up to this capacity build their lists with a warp for a few
+// particles (sph_warp.cu), larger ones with a thread per particle; measured,
+// thread / warp, event-timed: DFSPH rho + alpha + first divergence sweep 1 k
+// particles 52 / 14 us, 8 k 54 / 25, 27 k 57 / 41, 64 k 66 / 66, 125 k
+// - / 114 (thread 85); lists only 1 k 44 / 10, 64 k 54 / 37; WCSPH (4 threads
+// per particle) 27 k 34 / 31, 64 k 55 / 51
+constexpr int WARP_BUILD_MAX = 65536;
 void fill_solver_const(sphgpu_scene* h) {
     const SphParams& P = h->P;
     SolverConst& c = h->c;
@@ -286,6 +295,7 @@ void fill_solver_const(sphgpu_scene* h) {
     c.th_r = P.th_r;
     c.th_bt = P.th_bt;
     c.cap = h->ncap;
+    c.build = h->ncap <= 48 && (h->build < 0 ? h->cap <= WARP_BUILD_MAX : h->build != 0);
     c.stride = h->stride;
     c.l2pol = h->l2pol;
     c.lanes = h->wc_lanes ? h->wc_lanes : (h->cap <= (1 << 18) ? 4 : 1);
@@ -1358,6 +1368,7 @@ static int create_impl(const SphParams* p, int device, int max_fluid, int nscene
     fill_solver_const(h);
     mlp_init_attributes();
     ws_init_attributes();
+    warp_build_init();
     int r = alloc_scene(h);
     if (!r && nscenes > 1) {
         // per-scene state: grids, then one block for the BatchDev arrays
@@ -2904,6 +2915,7 @@ int sphgpu_get_solid_force(sphgpu_t h, int solid_id, double force[3], double tor
 //   carveout_sweeps/_build preferred L1/shared split of the sweeps / list build
 //   l2_policy              L2 eviction priorities of the sweeps' list and record loads
 //   fuse_div               DFSPH: the list build runs the divergence loop's first sweep A
+//   build                  list build (-1 by size, 0 a thread per particle, 1 a warp for a few)
 //   fuse_ws                warm start: feature gather and network in one kernel
 //   speculative_host_step  sphgpu_step_host runs part 1 while checking its inputs
 //   wc_lanes               WCSPH threads per particle (0 by size, 1, 4)
@@ -2913,6 +2925,12 @@ int sphgpu_debug_set(sphgpu_t h, const char* key, int value) {
     if (k == "record_kappa_sum") { h->record_ksum = value; invalidate_graphs(h); return 0; }
     if (k == "use_graphs") { h->use_graphs = value != 0; return 0; }
     if (k == "fuse_div") { h->fuse_div = value != 0; invalidate_graphs(h); return 0; }
+    if (k == "build") {
+        h->build = value;
+        fill_solver_const(h);
+        invalidate_graphs(h);
+        return 0;
+    }
     if (k == "fuse_ws") { h->fuse_ws = value != 0; invalidate_graphs(h); return 0; }
     if (k == "wc_lanes") {
         if (value != 0 && value != 1 && value != 4) return SPHGPU_EINVAL;

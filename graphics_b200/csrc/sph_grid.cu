@@ -19,7 +19,7 @@
 // entries a 48-cap truncates) are the reference's.  The cut test uses
 // round-to-nearest float ops in the reference's evaluation order, so the
 // neighbour sets are bit-identical.
-#include "sph_kernels.cuh"
+#include "sph_build.cuh"
 
 namespace {
 constexpr int NT = 256;
@@ -115,16 +115,15 @@ __global__ void __launch_bounds__(NT) k_rank_reorder(DevScene s, int dead_key, i
     if (carry & 8) s.cC[p] = s.cC_s[i];
 }
 
-__global__ void k_count_active(DevScene s, int dead_key) {
-    int staged = s.st->pad0;
-    int act = s.cell_start[dead_key];
-    s.st->removed += staged - act;
-    s.st->n_active = act;
-}
-
 // interleaved {fluid start, boundary start} per cell key: one 8-byte load
 // per cell bound in the neighbour-list kernel
-__global__ void k_merge_starts(DevScene s, int nk) {
+// dead_key >= 0: also the number of active particles
+__global__ void k_merge_starts(DevScene s, int nk, int dead_key) {
+    if (dead_key >= 0 && blockIdx.x == 0 && threadIdx.x == 0) {
+        const int staged = s.st->pad0, act = s.cell_start[dead_key];
+        s.st->removed += staged - act;
+        s.st->n_active = act;
+    }
     const int k = blockIdx.x * NT + threadIdx.x;
     if (k <= nk) s.cstart2[k] = make_int2(s.cell_start[k], s.bcell_start[k]);
 }
@@ -134,17 +133,7 @@ __global__ void k_merge_starts(DevScene s, int nk) {
 // spreads the rows of 8 consecutive threads over distinct bank quads).
 constexpr int LROW = 52;
 
-// mode 0: neighbour lists only; 1: + DFSPH rho and alpha
-// (DF_constantDensitySolverFirst, DFSPH.cpp:84-193); 2: + WCSPH rho and Tait
-// pressure (WcSph::wc_computePressure, WcSph.cpp:99-153); 3: + IISph
-// sphDensity, gamma, sphVolume and alpha (IISph.cpp:100-402); 4: mode 1 and,
-// over the same list in the same pass, the first sweep A of the divergence
-// loop that follows the neighbour search (DFSPH.cpp:795-835: Drho/Dt, its
-// clamp, kappa_v, the FP64 error sum) -- every neighbour's 32-byte
-// {position, velocity} record is gathered once for both, and the loop then
-// starts with its velocity update (the per-pair term is div_term, the one the
-// separate sweep uses, so the results are the same bit for bit); 5: mode 4 in
-// a batch (each scene's own dt; the loop decisions reduce per scene).
+// Modes: see sph_build.cuh.
 //
 // STAGED (cap <= 48): a kept neighbour is one predicated shared-memory store
 // into the thread's row -- no divergent branch around a global store in the
@@ -156,7 +145,6 @@ constexpr int LROW = 52;
 // occupancy leaves (60 instead of 48 with spills: 529 -> 520 us at 1 M).
 template <int MODE, int BS, bool STAGED>
 __global__ void __launch_bounds__(BS, STAGED ? 1024 / BS : 1) k_build(DevScene s, GridGeom g, SolverConst c) {
-    constexpr bool DIV = MODE == 4 || MODE == 5;  // the fused first divergence sweep
     extern __shared__ int4 list_smem[];
     int* const row = reinterpret_cast<int*>(list_smem) + (STAGED ? threadIdx.x * LROW : 0);
     const int n = s.st->n_active;
@@ -166,8 +154,6 @@ __global__ void __launch_bounds__(BS, STAGED ? 1024 / BS : 1) k_build(DevScene s
     const bool act = p < n;
     if (act) {
         const float4 pa = s.pos[p];
-        const int ph = phase_of(pa);
-        const float fm0 = c.fm_ph[ph], rho0 = c.rho0_ph[ph];
         const float4* __restrict__ P = s.pos;
         const float4* __restrict__ BP = s.bpos;
         const GridGeom G = s.nscenes > 1 ? s.b.geom[scene_of(pa)] : g;
@@ -226,95 +212,14 @@ __global__ void __launch_bounds__(BS, STAGED ? 1024 / BS : 1) k_build(DevScene s
             for (int gi = 0; gi < ((cnt + 3) >> 2); ++gi) o4[(size_t)gi * stride + p] = r4[gi];
         }
         s.ncount[p] = cnt;
-        if (MODE == 3) {
-            // IISph: sphDensity (DF_prepareAttribute, IISph.cpp:127-170) and
-            // VF_prepareAttribute (IISph.cpp:309-402) over the stored list,
-            // per-pair h = (d_a + d_b)/2 = d (one diameter for all particles)
-            const float Va = c.iv_V, ma = c.iv_m[ph], rda = rho0;
-            const float w0 = c.kd.theta;  // W(0, d)
-            float density = w0 * ma;
-            float gamma = Va * w0;
-            float sphv = (float)((double)w0 * (double)Va * (double)Va);
-            float a1x = 0.f, a1y = 0.f, a1z = 0.f, a2 = 0.f;
-            for (int k = 0; k < cnt; ++k) {
-                const unsigned e = STAGED ? (unsigned)row[k] : (unsigned)out[ell_index(stride, p, k)];
-                const bool bnd = (e & BND_FLAG) != 0u;
-                const float4 pb = __ldg((bnd ? BP : P) + (e & BND_MASK));
-                const float xx = pa.x - pb.x, xy = pa.y - pb.y, xz = pa.z - pb.z;
-                const float len2 = dis_square_rn(pa.x, pa.y, pa.z, pb.x, pb.y, pb.z);
-                float w, f;
-                kernel_pair_rn(c.kd, len2, w, f);
-                const float Vb = bnd ? pb.w : Va;
-                density = fmaf(bnd ? rda * Vb : c.iv_m[phase_of(pb)], w, density);
-                gamma = fmaf(Vb, w, gamma);
-                sphv = fmaf(Va * Vb, w, sphv);
-                const float fv = f * Vb;
-                a1x = fmaf(xx, fv, a1x);
-                a1y = fmaf(xy, fv, a1y);
-                a1z = fmaf(xz, fv, a1z);
-                // V_b^2 |gradW|^2 / m_b: fluid neighbours only (boundary terms
-                // belong to dynamic solids, IISph.cpp:386-393)
-                if (!bnd) a2 = fmaf(fv * fv, len2 / c.iv_m[phase_of(pb)], a2);
-            }
-            float al = ((a1x * a1x + a1y * a1y + a1z * a1z) / ma + a2) / gamma;
-            if (al < 1.0e-10f) al = 1.0e-10f;
-            s.ivs[p] = make_float4(gamma, sphv, 1.f / al, density);
-        } else if (MODE != 0) {
-            // phase 2: rho and alpha over the stored list (all lanes busy)
-            float density = ker_W(c.k, 0.f) * fm0;
-            float a1x = 0.f, a1y = 0.f, a1z = 0.f, a2 = 0.f;
-            float dacc = 0.f;  // MODE 4: the divergence sum
-            const float4 va = DIV ? s.pv[2 * p + 1] : make_float4(0.f, 0.f, 0.f, 0.f);
-            for (int k = 0; k < cnt; ++k) {
-                const unsigned e = STAGED ? (unsigned)row[k] : (unsigned)out[ell_index(stride, p, k)];
-                const bool bnd = (e & BND_FLAG) != 0u;
-                float4 pb, vb;
-                // pv / bpv hold {the position (boundary: with its volume) of
-                // pos / bpos, the velocity}
-                if (DIV) ld_record32((bnd ? s.bpv : s.pv) + 2 * (size_t)(e & BND_MASK), pb, vb);
-                else pb = __ldg((bnd ? BP : P) + (e & BND_MASK));
-                if (DIV) dacc = div_term(c, pa, va, pb, vb, bnd, dacc);
-                const float xx = pa.x - pb.x, xy = pa.y - pb.y, xz = pa.z - pb.z;
-                const float len2 = dis_square_rn(pa.x, pa.y, pa.z, pb.x, pb.y, pb.z);
-                float w, f;
-                kernel_pair(c.k, len2, w, f);
-                const float m = bnd ? rho0 * pb.w : fm0;
-                density = fmaf(m, w, density);
-                if (MODE == 1 || DIV) {
-                    const float fm = f * m;
-                    a1x = fmaf(xx, fm, a1x);
-                    a1y = fmaf(xy, fm, a1y);
-                    a1z = fmaf(xz, fm, a1z);
-                    const float t = bnd ? 0.f : fm * sqrtf(len2);  // |gradW| m, fluid only (DFSPH.cpp:161)
-                    a2 = fmaf(t, t, a2);
-                }
-            }
-            if (MODE == 1 || DIV) {
-                s.rho[p] = density;
-                s.prv[2 * p] = make_float4(pa.x, pa.y, pa.z, density);
-                float al = a1x * a1x + a1y * a1y + a1z * a1z + a2;
-                if (al < 1.0e-6f) al = 1.0e-6f;
-                const float alpha = density / al;
-                s.alpha[p] = alpha;
-                if (DIV) {
-                    // the divergence loop's first sweep A, as k_df_div_a
-                    const float dt = MODE == 5 ? s.b.dt[scene_of(pa)] : *s.dt;
-                    float dd = dacc;
-                    if (dd < 0.f || (density + dd * dt) < c.rho0) dd = 0.f;  // DFSPH.cpp:829-832
-                    const float kv = dd * alpha / dt;                         // DFSPH.cpp:835
-                    s.pk[p] = make_float4(pa.x, pa.y, pa.z, kv / density);
-                    s.kappav[p] = kv;
-                    s.aux1[p] = dd;
-                    ddiv = (double)dd;
-                }
-            } else {
-                s.rho[p] = density;
-                // Tait, WcSph.cpp:142-146 (NEGLECT_NEGATIVE_PRESSURE)
-                float pr = c.wc_B * (powf(density / rho0, c.wc_gamma) - 1.f);
-                if (pr < 0.f) pr = 0.f;
-                s.kr[p] = pr;
-            }
-        }
+        list_terms<MODE>(s, c, p, pa, cnt, ddiv, [&](int k, bool& bnd, float4& pb, float4& vb) {
+            const unsigned e = STAGED ? (unsigned)row[k] : (unsigned)out[ell_index(stride, p, k)];
+            bnd = (e & BND_FLAG) != 0u;
+            // pv / bpv hold {the position (boundary: with its volume) of
+            // pos / bpos, the velocity}
+            if (build_has_div(MODE)) ld_record32((bnd ? s.bpv : s.pv) + 2 * (size_t)(e & BND_MASK), pb, vb);
+            else pb = __ldg((bnd ? BP : P) + (e & BND_MASK));
+        });
     }
     __shared__ int sh[BS / 32];
     int tot = block_sum_int<BS>(act ? cnt : 0, sh);
@@ -593,12 +498,11 @@ void launch_scatter_reorder(const DevScene& s, const GridGeom& g, int n_old, int
 }
 
 void launch_count_active(const DevScene& s, const GridGeom& g, cudaStream_t st) {
-    k_count_active<<<1, 1, 0, st>>>(s, g.nkeys - 1);
-    k_merge_starts<<<nblk(g.nkeys + 1, NT), NT, 0, st>>>(s, g.nkeys);
+    k_merge_starts<<<nblk(g.nkeys + 1, NT), NT, 0, st>>>(s, g.nkeys, g.nkeys - 1);
 }
 
 void launch_merge_starts(const DevScene& s, const GridGeom& g, cudaStream_t st) {
-    k_merge_starts<<<nblk(g.nkeys + 1, NT), NT, 0, st>>>(s, g.nkeys);
+    k_merge_starts<<<nblk(g.nkeys + 1, NT), NT, 0, st>>>(s, g.nkeys, -1);
 }
 
 template <int BS, bool STAGED>
@@ -655,6 +559,10 @@ void preload_build_kernels() {
 
 void launch_build(const DevScene& s, const GridGeom& g, const SolverConst& c, int mode, int n_max, cudaStream_t st,
                   int bs) {
+    if (c.build) {
+        launch_warp_build(s, g, c, mode, n_max, st, bs);
+        return;
+    }
     if (mode == 2 && c.lanes == 4 && c.cap <= LROW - 4) {
         // small scenes: 4 threads per particle (sizes measured: 27 k particles,
         // 54 -> 35 us; 8 threads per particle 40 us)

@@ -203,17 +203,23 @@ __device__ __forceinline__ bool finish_sum(double* partial, unsigned* ticket, do
 }
 
 // One pair's term of the DFSPH divergence sums, m_j gradW_ij . (v_i - v_j)
-// (DFSPH.cpp:589-617, 795-825), accumulated into acc: neighbour j's record
-// {pb = (x, y, z, volume or phase), vb = loop velocity}; boundary mass
-// rho0 * volume.  The Jacobi sweeps and the list build's fused first
-// divergence sweep share it, so both round the same way.
-__device__ __forceinline__ float div_term(const SolverConst& c, float4 pa, float4 va, float4 pb, float4 vb, bool bnd,
-                                          float acc) {
-    const float m = bnd ? c.rho0 * pb.w : c.fm0;
+// (DFSPH.cpp:589-617, 795-825) as the two factors t and m of its fma into
+// the sum: neighbour j's record {pb = (x, y, z, volume or phase), vb = loop
+// velocity}; boundary mass rho0 * volume.  The Jacobi sweeps and the list
+// build's fused first divergence sweep share it, so all round the same way.
+__device__ __forceinline__ void div_pair(const SolverConst& c, float4 pa, float4 va, float4 pb, float4 vb, bool bnd,
+                                         float& t, float& m) {
+    m = bnd ? c.rho0 * pb.w : c.fm0;
     const float xx = pa.x - pb.x, xy = pa.y - pb.y, xz = pa.z - pb.z;
     const float f = grad_over_r(c.k, xx * xx + xy * xy + xz * xz);
     const float dot = xx * (va.x - vb.x) + xy * (va.y - vb.y) + xz * (va.z - vb.z);
-    return fmaf(dot * f, m, acc);
+    t = dot * f;
+}
+__device__ __forceinline__ float div_term(const SolverConst& c, float4 pa, float4 va, float4 pb, float4 vb, bool bnd,
+                                          float acc) {
+    float t, m;
+    div_pair(c, pa, va, pb, vb, bnd, t, m);
+    return fmaf(t, m, acc);
 }
 
 // ---- neighbour search (sph_grid.cu) ----
@@ -222,11 +228,12 @@ __device__ __forceinline__ float div_term(const SolverConst& c, float4 pa, float
 void launch_hash(const DevScene& s, const GridGeom& g, int integrate, int n_old, cudaStream_t st);
 // carry: bit 0 hist, bit 1 cA, bit 2 cB, bit 3 cC (staging -> sorted)
 void launch_scatter_reorder(const DevScene& s, const GridGeom& g, int n_old, int carry, cudaStream_t st);
+// active count and the interleaved cell starts
 void launch_count_active(const DevScene& s, const GridGeom& g, cudaStream_t st);
-// mode 0: lists only; 1: lists + DFSPH rho/alpha; 2: lists + WCSPH rho/pressure;
-// 3: lists + IISph VF_prepareAttribute / sphDensity (ivs); 4: mode 1 + the
-// divergence loop's first sweep A (Drho/Dt, kappa_v, and for a single scene
-// the FP64 error; a batch runs it with each scene's dt)
+// ---- list build, a warp per particle (sph_warp.cu) ----
+void launch_warp_build(const DevScene& s, const GridGeom& g, const SolverConst& c, int mode, int n_max, cudaStream_t st,
+                       int bs);
+void warp_build_init();
 void launch_build(const DevScene& s, const GridGeom& g, const SolverConst& c, int mode, int n_max, cudaStream_t st,
                   int bs = 128);
 void launch_to_ref_order(const float4* src, const int* gid, int n, float* dst3, cudaStream_t st);
