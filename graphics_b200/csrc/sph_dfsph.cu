@@ -61,72 +61,103 @@ __global__ void k_loop_reset(DevScene s, int which) {
 // before the current group's record gathers) and each neighbour costs one
 // 32-byte record; the per-pair divisions become reciprocals (1/rho_i once
 // per particle, 1/rho_j and 1/(r^2 + 0.01 h^2) per pair).
+struct ForceOwn {
+    float4 pa, va;
+    float dt, rhoa, bm, den0, visc, ax, ay, az;
+};
+__device__ __forceinline__ void force_begin(const DevScene& s, const SolverConst& c, int p, ForceOwn& o) {
+    o.pa = s.pos[p];
+    o.dt = dt_of(s, o.pa);
+    o.va = s.vel[p];
+    o.rhoa = s.rho[p];
+    o.bm = c.rho0 * __frcp_rn(o.rhoa);  // (frho0*volume)/fa.density = bm * volume, DFSPH.cpp:1353
+    o.den0 = 0.01f * c.hs * c.hs;
+    o.visc = 10.f * c.nu;
+    o.ax = c.gravity[0];
+    o.ay = c.gravity[1];
+    o.az = c.gravity[2];
+}
+// one neighbour's record {(x, y, z, rho), v} or, for a boundary particle,
+// {(x, y, z, volume), singleVelocity + velocity} (DFSPH.cpp:1349): the
+// factors (x, y, z) and w of its fma into the acceleration; false (w 0) if
+// the pair has no force
+__device__ __forceinline__ bool force_pair(const SolverConst& c, const ForceOwn& o, float4 pb, float4 vb, bool bnd,
+                                           int& zero, float4& f) {
+    const float m = bnd ? o.bm * pb.w               // DFSPH.cpp:1353
+                        : c.fm0 * __frcp_rn(pb.w);  // fm0/fb.density, DFSPH.cpp:1265
+    f.x = o.pa.x - pb.x;
+    f.y = o.pa.y - pb.y;
+    f.z = o.pa.z - pb.z;
+    f.w = 0.f;
+    const float len2 = f.x * f.x + f.y * f.y + f.z * f.z;
+    const bool z0 = len2 == 0.f;  // zero distance: counted, no force (m_EC.zeroDis)
+    zero += z0;
+    const float pro = (o.va.x - vb.x) * f.x + (o.va.y - vb.y) * f.y + (o.va.z - vb.z) * f.z;
+    if (z0 || !(pro < 0.f)) return false;
+    f.w = grad_over_r(c.k, len2) * pro * __frcp_rn(len2 + o.den0) * m * o.visc;
+    return true;
+}
+__device__ __forceinline__ void force_term(const SolverConst& c, ForceOwn& o, float4 pb, float4 vb, bool bnd, bool ok,
+                                           int& zero) {
+    float4 f;
+    int z = 0;
+    const bool on = force_pair(c, o, pb, vb, bnd, z, f);
+    if (ok) zero += z;
+    if (ok && on) {
+        o.ax = fmaf(f.x, f.w, o.ax);
+        o.ay = fmaf(f.y, f.w, o.ay);
+        o.az = fmaf(f.z, f.w, o.az);
+    }
+}
+// over the list, by one thread: entries past the count read the particle's own
+// record and are masked out
+__device__ __forceinline__ void force_sweep(const DevScene& s, const SolverConst& c, int p, ForceOwn& o, int& zero) {
+    const int cnt = s.ncount[p];
+    const int ng = (cnt + 3) >> 2;
+    const size_t stride = (size_t)c.stride;
+    const unsigned long long polL = l2_policy(c.l2pol & 3);  // lists stream through L2
+    int4 nxt = ng ? ell_group_pol(s.nbr, stride, p, 0, polL) : make_int4(0, 0, 0, 0);
+    for (int gi = 0; gi < ng; ++gi) {
+        const int4 cur = nxt;
+        if (gi + 1 < ng) nxt = ell_group_pol(s.nbr, stride, p, gi + 1, polL);
+        const unsigned e[4] = {(unsigned)cur.x, (unsigned)cur.y, (unsigned)cur.z, (unsigned)cur.w};
+        float4 pb[4], vb[4];
+        bool ok[4], bnd[4];
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            ok[t] = gi * 4 + t < cnt;
+            const unsigned u = ok[t] ? e[t] : (unsigned)p;
+            bnd[t] = (u & BND_FLAG) != 0u;
+            ld_record32((bnd[t] ? s.bpf : s.prv) + 2 * (size_t)(u & BND_MASK), pb[t], vb[t]);
+        }
+#pragma unroll
+        for (int t = 0; t < 4; ++t) force_term(c, o, pb[t], vb[t], bnd[t], ok[t], zero);
+    }
+}
+__device__ __forceinline__ void force_finish(const DevScene& s, const SolverConst& c, int p, const ForceOwn& o,
+                                             int warm) {
+    s.acc[p] = make_float4(o.ax, o.ay, o.az, 0.f);
+    // w: the previous step's predicted stiffness (warm-start history),
+    // which the feature sweep then reads with the neighbour's record
+    s.pv[2 * p + 1] = make_float4(o.va.x + o.ax * o.dt, o.va.y + o.ay * o.dt, o.va.z + o.az * o.dt, s.hist[p].x);
+    if (warm) {
+        // learned warm start: the predicted stiffness is applied once before
+        // the Jacobi loop as a pressure-velocity correction of the form of
+        // DFSPH.cpp:674 (launch_df_warm_correction with kappa/rho =
+        // kwarm/rho); the unmodified loop then runs to the same tolerance.
+        s.pk[p].w = s.kwarm[p] / o.rhoa;
+    }
+}
 template <int BS>
 __global__ void __launch_bounds__(BS) k_df_forces(DevScene s, SolverConst c, int warm) {
     const int n = s.st->n_active;
     const int p = blockIdx.x * BS + threadIdx.x;
     int zero = 0;
     if (p < n) {
-        const float4 pa = s.pos[p];
-        const float dt = dt_of(s, pa);
-        const float4 va = s.vel[p];
-        const float rhoa = s.rho[p];
-        const float fm0 = c.fm0;
-        const float bm = c.rho0 * __frcp_rn(rhoa);  // (frho0*volume)/fa.density = bm * volume, DFSPH.cpp:1353
-        const float den0 = 0.01f * c.hs * c.hs;
-        const float visc = 10.f * c.nu;
-        float ax = c.gravity[0], ay = c.gravity[1], az = c.gravity[2];
-        const int cnt = s.ncount[p];
-        const int ng = (cnt + 3) >> 2;
-        const size_t stride = (size_t)c.stride;
-        const unsigned long long polL = l2_policy(c.l2pol & 3);  // lists stream through L2
-        int4 nxt = ng ? ell_group_pol(s.nbr, stride, p, 0, polL) : make_int4(0, 0, 0, 0);
-        for (int gi = 0; gi < ng; ++gi) {
-            const int4 cur = nxt;
-            if (gi + 1 < ng) nxt = ell_group_pol(s.nbr, stride, p, gi + 1, polL);
-            const unsigned e[4] = {(unsigned)cur.x, (unsigned)cur.y, (unsigned)cur.z, (unsigned)cur.w};
-            // one 32-byte record per neighbour: {(x, y, z, rho), v} or, for a
-            // boundary particle, {(x, y, z, volume), singleVelocity + velocity}
-            // (DFSPH.cpp:1349); entries past the count read the particle's own
-            // record and are masked out
-            float4 pb[4], vb[4];
-            bool ok[4], bnd[4];
-#pragma unroll
-            for (int t = 0; t < 4; ++t) {
-                ok[t] = gi * 4 + t < cnt;
-                const unsigned u = ok[t] ? e[t] : (unsigned)p;
-                bnd[t] = (u & BND_FLAG) != 0u;
-                ld_record32((bnd[t] ? s.bpf : s.prv) + 2 * (size_t)(u & BND_MASK), pb[t], vb[t]);
-            }
-#pragma unroll
-            for (int t = 0; t < 4; ++t) {
-                const float m = bnd[t] ? bm * pb[t].w              // DFSPH.cpp:1353
-                                       : fm0 * __frcp_rn(pb[t].w);  // fm0/fb.density, DFSPH.cpp:1265
-                const float xx = pa.x - pb[t].x, xy = pa.y - pb[t].y, xz = pa.z - pb[t].z;
-                const float len2 = xx * xx + xy * xy + xz * xz;
-                const bool z0 = len2 == 0.f;  // zero distance: counted, no force (m_EC.zeroDis)
-                zero += ok[t] && z0;
-                const float pro = (va.x - vb[t].x) * xx + (va.y - vb[t].y) * xy + (va.z - vb[t].z) * xz;
-                if (ok[t] && !z0 && pro < 0.f) {
-                    const float f = grad_over_r(c.k, len2);
-                    const float tt = f * pro * __frcp_rn(len2 + den0) * m * visc;
-                    ax = fmaf(xx, tt, ax);
-                    ay = fmaf(xy, tt, ay);
-                    az = fmaf(xz, tt, az);
-                }
-            }
-        }
-        s.acc[p] = make_float4(ax, ay, az, 0.f);
-        // w: the previous step's predicted stiffness (warm-start history),
-        // which the feature sweep then reads with the neighbour's record
-        s.pv[2 * p + 1] = make_float4(va.x + ax * dt, va.y + ay * dt, va.z + az * dt, s.hist[p].x);
-        if (warm) {
-            // learned warm start: the predicted stiffness is applied once before
-            // the Jacobi loop as a pressure-velocity correction of the form of
-            // DFSPH.cpp:674 (launch_df_warm_correction with kappa/rho =
-            // kwarm/rho); the unmodified loop then runs to the same tolerance.
-            s.pk[p].w = s.kwarm[p] / rhoa;
-        }
+        ForceOwn o;
+        force_begin(s, c, p, o);
+        force_sweep(s, c, p, o, zero);
+        force_finish(s, c, p, o, warm);
     }
     if (__syncthreads_or(zero)) {
         if (zero) atomicAdd(&s.st->zero_dis, zero);
@@ -170,143 +201,217 @@ __device__ __forceinline__ float div_sweep(const DevScene& s, const SolverConst&
     return acc;
 }
 
-// density loop, part A: rho_adv, kappa, FP64 sum of rho_adv
+// what part A needs of its particle after the sum, loaded before it
+struct AOwn {
+    float rho, alpha, dt;
+    __device__ __forceinline__ void load(const DevScene& s, int p, float4 pa) {
+        rho = s.rho[p];
+        alpha = s.alpha[p];
+        dt = dt_of(s, pa);
+    }
+};
+// density loop, part A, after the sum: rho_adv, kappa; the particle's rho_adv
+__device__ __forceinline__ double dens_finish(const DevScene& s, const SolverConst& c, int p, const AOwn& o, float acc,
+                                              int record) {
+    const float rho0 = c.rho0;
+    const float rho = o.rho, dt = o.dt;
+    float dadv = fmaf(acc, dt, rho);
+    if (dadv < rho0) dadv = rho0;
+    // kappa = (rho_adv - rho0) / pow(dt,2) * alpha  (DFSPH.cpp:641)
+    const float kap = (float)((double)(dadv - rho0) / ((double)dt * (double)dt) * (double)o.alpha);
+    s.pk[p].w = kap / rho;
+    s.kappa[p] = kap;
+    if (record) s.ksum[p] += kap;
+    s.aux0[p] = dadv;
+    return (double)dadv;
+}
+// divergence loop, part A, after the sum: Drho/Dt, clamp, kappa_v
+__device__ __forceinline__ double div_finish(const DevScene& s, const SolverConst& c, int p, const AOwn& o, float acc) {
+    float dd = acc;
+    const float rho = o.rho, dt = o.dt;
+    if (dd < 0.f || (rho + dd * dt) < c.rho0) dd = 0.f;  // DFSPH.cpp:829-832
+    const float kv = dd * o.alpha / dt;                 // DFSPH.cpp:835
+    s.pk[p].w = kv / rho;
+    s.kappav[p] = kv;
+    s.aux1[p] = dd;
+    return (double)dd;
+}
+// the loop's FP64 error from the particles' total (no particle left, all
+// removed: nothing to solve)
+template <int DIV>
+__device__ __forceinline__ double a_mean(const SolverConst& c, int n, double tot) {
+    if (DIV) return n > 0 ? tot / (double)n : 0.0;
+    return n > 0 ? (tot / (double)n - (double)c.rho0) / (double)c.rho0 : 0.0;
+}
+// whether the loop goes on after iteration `it` (its error err: the mean
+// Drho/Dt, or the mean relative density error); status bits of a loop that
+// ends without its goal
+template <int DIV>
+__device__ __forceinline__ bool loop_goes_on(const SolverConst& c, double err, double dt, double goal_abs,
+                                             double goal_rel, int it, int min_it, int max_it, unsigned& status) {
+    if (DIV) {
+        const bool crit = goal_abs > 0 ? (err > goal_abs) : (err * dt / (double)c.rho0 > goal_rel);
+        const bool cont = (crit || it < min_it) && it <= max_it;
+        if (!cont && crit) status |= 2u;
+        return cont;
+    }
+    const bool crit = err > goal_rel;
+    bool cont = (crit || it < min_it) && it < max_it;
+    if (!cont && crit) status |= 1u;
+    if (!(err == err)) { cont = false; status |= 4u; }
+    return cont;
+}
+
+// The block's part of the loop's FP64 error sum.  Part B, whose decision
+// needs it, adds the blocks up (b_decide): a last block that waited for the
+// others would end every part A with a chain of a fence, an atomic and the
+// loads (about 3 us).  A batch reduces per scene (k_batch_decide).
 template <int BS>
-__global__ void __launch_bounds__(BS) k_df_dens_a(DevScene s, SolverConst c, int record) {
+__device__ __forceinline__ void a_partial(const DevScene& s, double mine) {
+    if (s.nscenes > 1) return;
+    __shared__ double sh[BS / 32];
+    const double b = block_sum_double<BS>(mine, sh);
+    if (threadIdx.x == 0) s.partial[blockIdx.x] = b;
+}
+
+// density loop, part A: rho_adv, kappa, FP64 sum of rho_adv.  Nine resident
+// blocks of 128 declared (56 registers: a group's four record gathers really
+// are in flight together; at 48, the compiler's choice before, they were
+// not).  With the sum's end moved to part B: 1 M particles 121 -> 103 us,
+// 216 k 42 -> 36, 69 k 19.6 -> 16.9 (event-timed).
+template <int BS>
+__global__ void __launch_bounds__(BS, 1152 / BS) k_df_dens_a(DevScene s, SolverConst c, int record) {
     const int n = s.st->n_active;
     const int p = blockIdx.x * BS + threadIdx.x;
     double mine = 0.0;
     if (p < n && scene_active(s, s.pv[2 * p])) {
         const float4 pa = s.pv[2 * p];
-        const float dt = dt_of(s, pa);
-        const float4 va = s.pv[2 * p + 1];
-        const float rho0 = c.rho0;
-        const float acc = div_sweep(s, c, p, pa, va);
-        const float rho = s.rho[p];
-        float dadv = fmaf(acc, dt, rho);
-        if (dadv < rho0) dadv = rho0;
-        // kappa = (rho_adv - rho0) / pow(dt,2) * alpha  (DFSPH.cpp:641)
-        const float kap = (float)((double)(dadv - rho0) / ((double)dt * (double)dt) * (double)s.alpha[p]);
-        s.pk[p].w = kap / rho;
-        s.kappa[p] = kap;
-        if (record) s.ksum[p] += kap;
-        s.aux0[p] = dadv;
-        mine = (double)dadv;
+        AOwn o;
+        o.load(s, p, pa);
+        mine = dens_finish(s, c, p, o, div_sweep(s, c, p, pa, s.pv[2 * p + 1]), record);
     }
-    if (s.nscenes > 1) return;  // a batch reduces per scene (k_batch_decide)
-    __shared__ double sh[BS / 32];
-    double bs = block_sum_double<BS>(mine, sh);
-    double tot;
-    if (finish_sum<BS>(s.partial, &s.st->ticket[0], bs, &tot)) {
-        // no particle left (all removed): nothing to solve
-        s.st->err_density = n > 0 ? (tot / (double)n - (double)c.rho0) / (double)c.rho0 : 0.0;
-    }
+    a_partial<BS>(s, mine);
 }
 
 // density/divergence loop, part B: v_adv update with k = kappa/rho
 // (DFSPH.cpp:647-693 / 840-883); then the loop decision.  Each neighbour
 // costs one 16-byte record (x, y, z, k) (pk; boundary: (x, y, z, volume)).
+// Nine resident blocks of 128 declared (40 registers and 73 us at 1 M
+// without, 54 and 62 us with; 68 us when the decision was a thread of the
+// first particle block).
+// one neighbour's factors (x, y, z) and w of its fma into the update
+__device__ __forceinline__ void v_pair(const SolverConst& c, float4 pa, float4 pb, bool bnd, float4& f) {
+    const float ka = pa.w;
+    const float fa = c.fm0 * ka, ba = c.rho0 * ka;
+    const float w = bnd ? ba * pb.w : fmaf(c.fm0, pb.w, fa);
+    f.x = pa.x - pb.x;
+    f.y = pa.y - pb.y;
+    f.z = pa.z - pb.z;
+    f.w = grad_over_r(c.k, f.x * f.x + f.y * f.y + f.z * f.z) * w;
+}
+__device__ __forceinline__ void v_term(const SolverConst& c, float4 pa, float4 pb, bool bnd, bool ok, float& dx,
+                                       float& dy, float& dz) {
+    float4 f;
+    v_pair(c, pa, pb, bnd, f);
+    if (!ok) f.w = 0.f;
+    dx = fmaf(f.x, f.w, dx);
+    dy = fmaf(f.y, f.w, dy);
+    dz = fmaf(f.z, f.w, dz);
+}
+__device__ __forceinline__ void v_sweep(const DevScene& s, const SolverConst& c, int p, float4 pa, float& dx, float& dy,
+                                        float& dz) {
+    const int cnt = s.ncount[p];
+    const int ng = (cnt + 3) >> 2;
+    const size_t stride = (size_t)c.stride;
+    const unsigned long long polL = l2_policy(c.l2pol & 3), polR = l2_policy((c.l2pol >> 2) & 3);
+    int4 nxt = ng ? ell_group_pol(s.nbr, stride, p, 0, polL) : make_int4(0, 0, 0, 0);
+    for (int gi = 0; gi < ng; ++gi) {
+        const int4 cur = nxt;
+        if (gi + 1 < ng) nxt = ell_group_pol(s.nbr, stride, p, gi + 1, polL);
+        const unsigned e[4] = {(unsigned)cur.x, (unsigned)cur.y, (unsigned)cur.z, (unsigned)cur.w};
+        float4 pb[4];
+        bool ok[4], bnd[4];
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            ok[t] = gi * 4 + t < cnt;
+            const unsigned u = ok[t] ? e[t] : (unsigned)p;
+            bnd[t] = (u & BND_FLAG) != 0u;
+            const unsigned j = u & BND_MASK;
+            pb[t] = ld_f4_pol(bnd[t] ? s.bpv + 2 * (size_t)j : s.pk + j, polR);
+        }
+#pragma unroll
+        for (int t = 0; t < 4; ++t) v_term(c, pa, pb[t], bnd[t], ok[t], dx, dy, dz);
+    }
+}
+template <int DIV>
+__device__ __forceinline__ void v_finish(const DevScene& s, int p, float4 va, float dt, float dx, float dy, float dz) {
+    va.x = fmaf(-dx, dt, va.x);
+    va.y = fmaf(-dy, dt, va.y);
+    va.z = fmaf(-dz, dt, va.z);
+    s.pv[2 * p + 1] = va;
+    if (DIV) {
+        s.vel[p] = va;  // velocity = vel_adv (DFSPH.cpp:909)
+        s.prv[2 * p + 1] = va;
+    }
+}
+// Part B's first block, which takes no particles: the error sum of part A's
+// `parts` blocks and the convergence decision of the iteration.
+template <int BS, int DIV>
+__device__ __forceinline__ void b_decide(const DevScene& s, const SolverConst& c, int parts, double goal_abs,
+                                         double goal_rel, int min_it, int max_it, cudaGraphConditionalHandle h,
+                                         int use_handle) {
+    __shared__ double sh[BS / 32];
+    const double tot = block_sum_double<BS>(partials_share<BS>(s.partial, parts), sh);
+    if (threadIdx.x != 0) return;
+    const double err = a_mean<DIV>(c, s.st->n_active, tot);
+    (DIV ? s.st->err_div : s.st->err_density) = err;
+    int it;
+    if (DIV) {
+        it = ++s.st->it_div;
+        ++s.st->total_it_div;
+    } else {
+        it = ++s.st->it_density;
+        ++s.st->total_it_density;
+    }
+    unsigned status = 0;
+    const int cont = loop_goes_on<DIV>(c, err, (double)*s.dt, goal_abs, goal_rel, it, min_it, max_it, status);
+    if (status) atomicOr(&s.st->status, status);
+    s.st->cont = cont;
+    if (use_handle) cudaGraphSetConditional(h, cont ? 1u : 0u);
+}
 template <int BS, int DIV, int DECIDE>
-__global__ void __launch_bounds__(BS) k_df_vupdate(DevScene s, SolverConst c, double goal_abs, double goal_rel,
+__global__ void __launch_bounds__(BS, 1152 / BS) k_df_vupdate(DevScene s, SolverConst c, int parts, double goal_abs, double goal_rel,
                                                    int min_it, int max_it, cudaGraphConditionalHandle h,
                                                    int use_handle) {
+    int bid = blockIdx.x;
+    if (DECIDE && parts && bid-- == 0) {
+        b_decide<BS, DIV>(s, c, parts, goal_abs, goal_rel, min_it, max_it, h, use_handle);
+        return;
+    }
     const int n = s.st->n_active;
-    const int p = blockIdx.x * BS + threadIdx.x;
+    const int p = bid * BS + threadIdx.x;
     if (p < n && scene_active(s, s.pv[2 * p])) {
         const float dt = dt_of(s, s.pv[2 * p]);
         const float4 pa = s.pk[p];
-        float4 va = s.pv[2 * p + 1];
-        const float ka = pa.w;
-        const float fa = c.fm0 * ka, ba = c.rho0 * ka;
         float dx = 0.f, dy = 0.f, dz = 0.f;
-        const int cnt = s.ncount[p];
-        const int ng = (cnt + 3) >> 2;
-        const size_t stride = (size_t)c.stride;
-        const unsigned long long polL = l2_policy(c.l2pol & 3), polR = l2_policy((c.l2pol >> 2) & 3);
-        int4 nxt = ng ? ell_group_pol(s.nbr, stride, p, 0, polL) : make_int4(0, 0, 0, 0);
-        for (int gi = 0; gi < ng; ++gi) {
-            const int4 cur = nxt;
-            if (gi + 1 < ng) nxt = ell_group_pol(s.nbr, stride, p, gi + 1, polL);
-            const unsigned e[4] = {(unsigned)cur.x, (unsigned)cur.y, (unsigned)cur.z, (unsigned)cur.w};
-            float4 pb[4];
-            bool ok[4], bnd[4];
-#pragma unroll
-            for (int t = 0; t < 4; ++t) {
-                ok[t] = gi * 4 + t < cnt;
-                const unsigned u = ok[t] ? e[t] : (unsigned)p;
-                bnd[t] = (u & BND_FLAG) != 0u;
-                const unsigned j = u & BND_MASK;
-                pb[t] = ld_f4_pol(bnd[t] ? s.bpv + 2 * (size_t)j : s.pk + j, polR);
-            }
-#pragma unroll
-            for (int t = 0; t < 4; ++t) {
-                const float w = bnd[t] ? ba * pb[t].w : fmaf(c.fm0, pb[t].w, fa);
-                const float xx = pa.x - pb[t].x, xy = pa.y - pb[t].y, xz = pa.z - pb[t].z;
-                const float f = ok[t] ? grad_over_r(c.k, xx * xx + xy * xy + xz * xz) * w : 0.f;
-                dx = fmaf(xx, f, dx);
-                dy = fmaf(xy, f, dy);
-                dz = fmaf(xz, f, dz);
-            }
-        }
-        va.x = fmaf(-dx, dt, va.x);
-        va.y = fmaf(-dy, dt, va.y);
-        va.z = fmaf(-dz, dt, va.z);
-        s.pv[2 * p + 1] = va;
-        if (DIV) {
-            s.vel[p] = va;  // velocity = vel_adv (DFSPH.cpp:909)
-            s.prv[2 * p + 1] = va;
-        }
-    }
-    if (DECIDE && s.nscenes <= 1 && blockIdx.x == 0 && threadIdx.x == 0) {
-        // convergence decision of the iteration that just finished
-        int it;
-        int cont;
-        if (DIV) {
-            it = ++s.st->it_div;
-            ++s.st->total_it_div;
-            const double avg = s.st->err_div;  // mean Drho/Dt of this iteration
-            const double dtd = (double)*s.dt;
-            bool crit = goal_abs > 0 ? (avg > goal_abs) : (avg * dtd / (double)c.rho0 > goal_rel);
-            cont = (crit || it < min_it) && it <= max_it;
-            if (!cont && crit) atomicOr(&s.st->status, 2u);
-        } else {
-            it = ++s.st->it_density;
-            ++s.st->total_it_density;
-            const double err = s.st->err_density;
-            bool crit = err > goal_rel;
-            cont = (crit || it < min_it) && it < max_it;
-            if (!cont && crit) atomicOr(&s.st->status, 1u);
-            if (!(err == err)) { cont = 0; atomicOr(&s.st->status, 4u); }
-        }
-        s.st->cont = cont;
-        if (use_handle) cudaGraphSetConditional(h, cont ? 1u : 0u);
+        v_sweep(s, c, p, pa, dx, dy, dz);
+        v_finish<DIV>(s, p, s.pv[2 * p + 1], dt, dx, dy, dz);
     }
 }
 
 // divergence loop, part A: Drho/Dt, clamp, kappa_v, FP64 sum
 template <int BS>
-__global__ void __launch_bounds__(BS) k_df_div_a(DevScene s, SolverConst c) {
+__global__ void __launch_bounds__(BS, 1152 / BS) k_df_div_a(DevScene s, SolverConst c) {
     const int n = s.st->n_active;
     const int p = blockIdx.x * BS + threadIdx.x;
     double mine = 0.0;
     if (p < n && scene_active(s, s.pv[2 * p])) {
         const float4 pa = s.pv[2 * p];
-        const float dt = dt_of(s, pa);
-        const float4 va = s.pv[2 * p + 1];
-        float dd = div_sweep(s, c, p, pa, va);
-        const float rho = s.rho[p];
-        if (dd < 0.f || (rho + dd * dt) < c.rho0) dd = 0.f;  // DFSPH.cpp:829-832
-        const float kv = dd * s.alpha[p] / dt;              // DFSPH.cpp:835
-        s.pk[p].w = kv / rho;
-        s.kappav[p] = kv;
-        s.aux1[p] = dd;
-        mine = (double)dd;
+        AOwn o;
+        o.load(s, p, pa);
+        mine = div_finish(s, c, p, o, div_sweep(s, c, p, pa, s.pv[2 * p + 1]));
     }
-    if (s.nscenes > 1) return;  // a batch reduces per scene (k_batch_decide)
-    __shared__ double sh[BS / 32];
-    double bs = block_sum_double<BS>(mine, sh);
-    double tot;
-    if (finish_sum<BS>(s.partial, &s.st->ticket[1], bs, &tot)) s.st->err_div = n > 0 ? tot / (double)n : 0.0;
+    a_partial<BS>(s, mine);
 }
 
 // FP64 max |v| and the CFL step dt = clamp(cfl * d / vmax, dt_min, dt_max).
@@ -344,7 +449,13 @@ __global__ void __launch_bounds__(NT) k_cfl(DevScene s, float cfl, float d, floa
     __threadfence();
     // the last block reduces the block maxima with all its threads
     double vm = 0;
-    for (int i = threadIdx.x; i < (int)gridDim.x; i += NT) vm = fmax(vm, ((volatile double*)s.partial)[i]);
+    for (int i0 = threadIdx.x; i0 < (int)gridDim.x; i0 += 8 * NT) {
+        double v[8];  // eight loads in flight (see partials_share)
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v[k] = i0 + k * NT < (int)gridDim.x ? __ldcg(s.partial + i0 + k * NT) : 0.0;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) vm = fmax(vm, v[k]);
+    }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) vm = fmax(vm, __shfl_down_sync(0xffffffffu, vm, o));
     __syncthreads();
@@ -384,22 +495,32 @@ void launch_df_forces(const DevScene& s, const SolverConst& c, int n_max, int wa
 void launch_df_dens_a(const DevScene& s, const SolverConst& c, int n_max, int record, cudaStream_t st, int bs) {
     DISPATCH_BS(bs, (k_df_dens_a<B><<<nblk(n_max, B), B, 0, st>>>(s, c, record)));
 }
-void launch_df_dens_b(const DevScene& s, const SolverConst& c, int n_max, double goal, int min_it, int max_it,
+int df_a_blocks(const SolverConst& c, int n_max, int bs) {
+    return nblk(n_max, bs == 64 || bs == 256 ? bs : 128);
+}
+template <int DIV, int DECIDE>
+static void launch_df_b(const DevScene& s, const SolverConst& c, int n_max, int parts, double goal_abs, double goal_rel,
+                        int min_it, int max_it, unsigned long long cond_handle, int use_handle, cudaStream_t st,
+                        int bs) {
+    const cudaGraphConditionalHandle h = (cudaGraphConditionalHandle)cond_handle;
+    if (s.nscenes > 1) parts = 0;  // a batch decides per scene
+    const int extra = DECIDE && parts ? 1 : 0;
+    DISPATCH_BS(bs, (k_df_vupdate<B, DIV, DECIDE><<<nblk(n_max, B) + extra, B, 0, st>>>(
+                        s, c, parts, goal_abs, goal_rel, min_it, max_it, h, use_handle)));
+}
+void launch_df_dens_b(const DevScene& s, const SolverConst& c, int n_max, int parts, double goal, int min_it, int max_it,
                       unsigned long long cond_handle, int use_handle, cudaStream_t st, int bs) {
-    DISPATCH_BS(bs, (k_df_vupdate<B, 0, 1><<<nblk(n_max, B), B, 0, st>>>(
-                        s, c, 0.0, goal, min_it, max_it, (cudaGraphConditionalHandle)cond_handle, use_handle)));
+    launch_df_b<0, 1>(s, c, n_max, parts, 0.0, goal, min_it, max_it, cond_handle, use_handle, st, bs);
 }
 void launch_df_warm_correction(const DevScene& s, const SolverConst& c, int n_max, cudaStream_t st, int bs) {
-    DISPATCH_BS(bs, (k_df_vupdate<B, 0, 0><<<nblk(n_max, B), B, 0, st>>>(s, c, 0.0, 0.0, 0, 0,
-                                                                         (cudaGraphConditionalHandle)0, 0)));
+    launch_df_b<0, 0>(s, c, n_max, 0, 0.0, 0.0, 0, 0, 0ull, 0, st, bs);
 }
 void launch_df_div_a(const DevScene& s, const SolverConst& c, int n_max, cudaStream_t st, int bs) {
     DISPATCH_BS(bs, (k_df_div_a<B><<<nblk(n_max, B), B, 0, st>>>(s, c)));
 }
-void launch_df_div_b(const DevScene& s, const SolverConst& c, int n_max, double goal_abs, double goal_rel,
+void launch_df_div_b(const DevScene& s, const SolverConst& c, int n_max, int parts, double goal_abs, double goal_rel,
                      int min_it, int max_it, unsigned long long cond_handle, int use_handle, cudaStream_t st, int bs) {
-    DISPATCH_BS(bs, (k_df_vupdate<B, 1, 1><<<nblk(n_max, B), B, 0, st>>>(
-                        s, c, goal_abs, goal_rel, min_it, max_it, (cudaGraphConditionalHandle)cond_handle, use_handle)));
+    launch_df_b<1, 1>(s, c, n_max, parts, goal_abs, goal_rel, min_it, max_it, cond_handle, use_handle, st, bs);
 }
 // every block-size instantiation of the per-neighbour sweep kernels
 template <int B, class F>

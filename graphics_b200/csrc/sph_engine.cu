@@ -531,7 +531,7 @@ int enq_df_density_loop(sphgpu_scene* h, bool capturing) {
         launch(h, "df_density_a", st,
                [&] { launch_df_dens_a(d, h->c, h->cap, h->record_ksum, st, h->tune.sweep_a); });
         launch(h, "df_density_b", st, [&] {
-            launch_df_dens_b(d, h->c, h->cap, P.df_density_goal, P.df_density_min_iter, P.df_density_max_iter, hd,
+            launch_df_dens_b(d, h->c, h->cap, df_a_blocks(h->c, h->cap, h->tune.sweep_a), P.df_density_goal, P.df_density_min_iter, P.df_density_max_iter, hd,
                              use, st, h->tune.sweep_b);
         });
         if (h->nscenes > 1)
@@ -549,9 +549,9 @@ int enq_df_div_loop(sphgpu_scene* h, bool capturing, bool fused = false) {
     launch_df_loop_reset(d, 1, h->stream);
     if (h->nscenes > 1) launch_batch_loop_reset(d, h->nscenes, 1, h->stream);
     // the velocity update and, for a batch, the per-scene decisions
-    auto div_b = [&](cudaStream_t st, unsigned long long hd, int use) {
+    auto div_b_of = [&](int parts, cudaStream_t st, unsigned long long hd, int use) {
         launch(h, "df_div_b", st, [&] {
-            launch_df_div_b(d, h->c, h->cap, P.df_div_goal_abs, P.df_div_goal_rel, P.df_div_min_iter,
+            launch_df_div_b(d, h->c, h->cap, parts, P.df_div_goal_abs, P.df_div_goal_rel, P.df_div_min_iter,
                             P.df_div_max_iter, hd, use, st, h->tune.sweep_b);
         });
         if (h->nscenes > 1)
@@ -562,9 +562,12 @@ int enq_df_div_loop(sphgpu_scene* h, bool capturing, bool fused = false) {
     };
     auto body = [&](cudaStream_t st, unsigned long long hd, int use) {
         launch(h, "df_div_a", st, [&] { launch_df_div_a(d, h->c, h->cap, st, h->tune.sweep_a); });
-        div_b(st, hd, use);
+        div_b_of(df_a_blocks(h->c, h->cap, h->tune.sweep_a), st, hd, use);
     };
-    return enq_loop(h, capturing, body, div_b, fused);
+    auto first_b = [&](cudaStream_t st, unsigned long long hd, int use) {
+        div_b_of(build_blocks(h->c, h->cap, h->tune.build), st, hd, use);
+    };
+    return enq_loop(h, capturing, body, first_b, fused);
 }
 
 // the list build runs the divergence loop's first sweep A

@@ -231,12 +231,11 @@ __global__ void __launch_bounds__(BS, STAGED ? 1024 / BS : 1) k_build(DevScene s
         if (mx) atomicMax(&s.st->max_nbrs, mx);
     }
     if (MODE == 4) {
-        // mean Drho/Dt of the iteration (k_df_div_a's FP64 error; a batch,
-        // mode 5, reduces per scene in k_batch_decide)
+        // the block's part of the iteration's FP64 sum of Drho/Dt (as
+        // k_df_div_a; a batch, mode 5, reduces per scene in k_batch_decide)
         __shared__ double shd[BS / 32];
         const double bsum = block_sum_double<BS>(ddiv, shd);
-        double t;
-        if (finish_sum<BS>(s.partial, &s.st->ticket[1], bsum, &t)) s.st->err_div = n > 0 ? t / (double)n : 0.0;
+        if (threadIdx.x == 0) s.partial[blockIdx.x] = bsum;
     }
 }
 
@@ -573,6 +572,11 @@ void launch_build(const DevScene& s, const GridGeom& g, const SolverConst& c, in
     if (bs == 64) launch_build_bs<64>(s, g, c, mode, n_max, st);
     else if (bs == 256) launch_build_bs<256>(s, g, c, mode, n_max, st);
     else launch_build_bs<128>(s, g, c, mode, n_max, st);
+}
+
+int build_blocks(const SolverConst& c, int n_max, int bs) {
+    if (c.build) return warp_build_blocks(n_max, bs);
+    return nblk(n_max > 0 ? n_max : 1, bs == 64 || bs == 256 ? bs : 128);
 }
 
 void launch_boundary_keys(const float4* bpos, int nb, const GridGeom& g, int* keys, cudaStream_t st) {

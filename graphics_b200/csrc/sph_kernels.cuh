@@ -176,6 +176,24 @@ __device__ __forceinline__ bool scene_active(const DevScene& s, float4 pa) {
     return s.nscenes <= 1 || s.b.active[scene_of(pa)] != 0;
 }
 
+// This thread's share of the sum of n per-block partials, every BS-th in
+// order: loads through L2 (the blocks wrote them moments ago), eight in
+// flight -- one at a time each waits out the L2 latency (7813 partials by 128
+// threads: about 20 us at the end of a sweep).
+template <int BS>
+__device__ __forceinline__ double partials_share(const double* partial, int n) {
+    double acc = 0.0;
+    for (int i0 = threadIdx.x; i0 < n; i0 += 8 * BS) {
+        double v[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v[k] = i0 + k * BS < n ? __ldcg(partial + i0 + k * BS) : 0.0;
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+            if (i0 + k * BS < n) acc += v[k];
+    }
+    return acc;
+}
+
 // last-block FP64 reduction of per-block partials; returns true in the
 // thread that holds the total (thread 0 of the last block).  The partials
 // are summed in block order, so the total is the same from run to run.
@@ -192,9 +210,7 @@ __device__ __forceinline__ bool finish_sum(double* partial, unsigned* ticket, do
     if (!last) return false;
     __threadfence();
     __shared__ double sh[BS / 32];
-    double acc = 0;
-    for (int i = threadIdx.x; i < (int)gridDim.x; i += BS) acc += ((volatile double*)partial)[i];
-    double tot = block_sum_double<BS>(acc, sh);
+    double tot = block_sum_double<BS>(partials_share<BS>(partial, (int)gridDim.x), sh);
     if (threadIdx.x == 0) {
         *total = tot;
         *ticket = 0u;
@@ -233,6 +249,7 @@ void launch_count_active(const DevScene& s, const GridGeom& g, cudaStream_t st);
 // ---- list build, a warp per particle (sph_warp.cu) ----
 void launch_warp_build(const DevScene& s, const GridGeom& g, const SolverConst& c, int mode, int n_max, cudaStream_t st,
                        int bs);
+int warp_build_blocks(int n_max, int bs);
 void warp_build_init();
 void launch_build(const DevScene& s, const GridGeom& g, const SolverConst& c, int mode, int n_max, cudaStream_t st,
                   int bs = 128);
@@ -259,10 +276,14 @@ void launch_boundary_volume(const DevScene& s, const GridGeom& g, float dpart, f
 // bs: threads per block (64, 128 or 256; the autotuner's choice)
 void launch_df_forces(const DevScene& s, const SolverConst& c, int n_max, int warm, cudaStream_t st, int bs = 128);
 void launch_df_dens_a(const DevScene& s, const SolverConst& c, int n_max, int record, cudaStream_t st, int bs = 128);
-void launch_df_dens_b(const DevScene& s, const SolverConst& c, int n_max, double goal, int min_it, int max_it,
+// blocks of part A (or of the list build with the first divergence sweep):
+// the FP64 partials that part B's decision adds up (its `parts`)
+int df_a_blocks(const SolverConst& c, int n_max, int bs);
+int build_blocks(const SolverConst& c, int n_max, int bs);
+void launch_df_dens_b(const DevScene& s, const SolverConst& c, int n_max, int parts, double goal, int min_it, int max_it,
                       unsigned long long cond_handle, int use_handle, cudaStream_t st, int bs = 128);
 void launch_df_div_a(const DevScene& s, const SolverConst& c, int n_max, cudaStream_t st, int bs = 128);
-void launch_df_div_b(const DevScene& s, const SolverConst& c, int n_max, double goal_abs, double goal_rel,
+void launch_df_div_b(const DevScene& s, const SolverConst& c, int n_max, int parts, double goal_abs, double goal_rel,
                      int min_it, int max_it, unsigned long long cond_handle, int use_handle, cudaStream_t st,
                      int bs = 128);
 void launch_df_warm_correction(const DevScene& s, const SolverConst& c, int n_max, cudaStream_t st, int bs = 128);

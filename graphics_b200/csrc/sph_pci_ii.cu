@@ -69,9 +69,18 @@ __device__ __forceinline__ bool finish_sum2(double* partial, unsigned* ticket, d
     __threadfence();
     __shared__ double sh[NT / 32];
     double x = 0, y = 0;
-    for (int i = threadIdx.x; i < (int)gridDim.x; i += NT) {
-        x += ((volatile double*)partial)[2 * i];
-        y += ((volatile double*)partial)[2 * i + 1];
+    for (int i0 = threadIdx.x; i0 < (int)gridDim.x; i0 += 8 * NT) {
+        double2 v[8];  // eight loads in flight (see partials_share)
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+            v[k] = i0 + k * NT < (int)gridDim.x ? __ldcg(reinterpret_cast<const double2*>(partial) + i0 + k * NT)
+                                                : make_double2(0.0, 0.0);
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+            if (i0 + k * NT < (int)gridDim.x) {
+                x += v[k].x;
+                y += v[k].y;
+            }
     }
     double tx = block_sum_double<NT>(x, sh);
     double ty = block_sum_double<NT>(y, sh);

@@ -231,25 +231,28 @@ __global__ void __launch_bounds__(BS) k_warp_build(const __grid_constant__ DevSc
         if (mx) atomicMax(&s.st->max_nbrs, mx);
     }
     if (MODE == 4) {
-        // mean Drho/Dt of the iteration (k_df_div_a's FP64 error; a batch,
-        // mode 5, reduces per scene in k_batch_decide)
+        // the block's part of the iteration's FP64 sum of Drho/Dt (as
+        // k_df_div_a; a batch, mode 5, reduces per scene in k_batch_decide)
         __shared__ double shd[WPB];
         const double bsum = block_sum_double<BS>(dsum, shd);
-        double t;
-        if (finish_sum<BS>(s.partial, &s.st->ticket[1], bsum, &t)) s.st->err_div = n > 0 ? t / (double)n : 0.0;
+        if (threadIdx.x == 0) s.partial[blockIdx.x] = bsum;
     }
 }
 }  // namespace
 
 #define EACH_MODE(DO) DO(0) DO(1) DO(2) DO(3) DO(4) DO(5)
 
+// particles per warp: enough warps for every SM first
+static int warp_group(int n_max) { return std::min(GROUP, std::max(1, n_max / (148 * 16))); }
+int warp_build_blocks(int n_max, int bs) {
+    const int per = (bs == 64 || bs == 256 ? bs : 128) / 32 * warp_group(n_max), n = n_max > 0 ? n_max : 1;
+    return (n + per - 1) / per;
+}
+
 void launch_warp_build(const DevScene& s, const GridGeom& g, const SolverConst& c, int mode, int n_max, cudaStream_t st,
                        int bs) {
     if (mode == 4 && s.nscenes > 1) mode = 5;
-    // enough warps for every SM first, then more particles per warp
-    const int wpb = (bs == 64 || bs == 256 ? bs : 128) / 32, n = n_max > 0 ? n_max : 1;
-    const int group = std::min(GROUP, std::max(1, n / (148 * 16)));
-    const int nb = (n + wpb * group - 1) / (wpb * group);
+    const int group = warp_group(n_max), nb = warp_build_blocks(n_max, bs);
 #define GO(M, B) k_warp_build<M, B><<<nb, B, sizeof(WarpSmem<M>) * (B / 32), st>>>(s, g, c, group)
 #define ONE(M)                          \
     case M:                             \
