@@ -414,6 +414,171 @@ __global__ void __launch_bounds__(BS, 1152 / BS) k_df_div_a(DevScene s, SolverCo
     a_partial<BS>(s, mine);
 }
 
+// ---- the sweeps with four threads per particle (small scenes) ----
+//
+// In a small scene one thread's serial walk over some 28 neighbours is the
+// time of the whole sweep, however few particles there are.  Here lane t of
+// a particle's four takes the entries t, t + 4, ... -- a list group is one
+// 16-byte read of four lanes -- and leaves each entry's factors in shared
+// memory; the sum then runs over them in list order, so the results are
+// those of one thread per particle bit for bit.  Event-timed, one thread /
+// four: A 1 k particles 13.2 / 11.9 us, 8 k 15.1 / 11.0, 22 k 14.9 / 12.6,
+// 47 k 15.2 / 17.5; B 4 k 10.2 / 8.7, 8 k 10.8 / 9.9, 16 k 10.6 / 10.7, 33 k
+// 10.7 / 12.6; forces 1 k 15.8 / 10.6, 22 k 16.8 / 13.1, 47 k 17.5 / 20.9.
+constexpr int LANES = 4;
+constexpr int LROWS = 52;  // entries per particle's row (cap <= 48): rows start 8 or 16 words apart modulo the banks
+
+// f(k, e, ok) for the lane's entries k, four of them unrolled together:
+// ld(i, e) loads the record of the i-th, use(i, k, e) takes it (k < cnt)
+template <class Ld, class Use>
+__device__ __forceinline__ void lane_entries(const DevScene& s, const SolverConst& c, int p, int t, int cnt, Ld&& ld,
+                                             Use&& use) {
+    const size_t stride = (size_t)c.stride;
+    for (int g0 = 0; 4 * g0 < cnt; g0 += 4) {
+        unsigned e[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            e[i] = (unsigned)p;
+            if (4 * (g0 + i) + t < cnt) e[i] = (unsigned)__ldg(s.nbr + ((size_t)(g0 + i) * stride + p) * 4 + t);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) ld(i, e[i]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (4 * (g0 + i) + t < cnt) use(i, 4 * (g0 + i) + t, e[i]);
+    }
+}
+
+// DIV 0: density loop, part A (k_df_dens_a); 1: divergence loop, part A
+// (k_df_div_a)
+template <int BS, int DIV>
+__global__ void __launch_bounds__(BS) k_df_a_lanes(DevScene s, SolverConst c, int record) {
+    __shared__ float2 term[BS / LANES][LROWS];
+    const int n = s.st->n_active;
+    const int t = threadIdx.x % LANES, q = threadIdx.x / LANES;
+    const int p = blockIdx.x * (BS / LANES) + q;
+    double mine = 0.0;
+    float4 pa;
+    AOwn o;
+    int cnt = 0;
+    bool act = p < n;
+    if (act) {
+        pa = s.pv[2 * p];
+        act = scene_active(s, pa);
+    }
+    if (act) {
+        o.load(s, p, pa);
+        const float4 va = s.pv[2 * p + 1];
+        cnt = s.ncount[p];
+        float4 pb[4], vb[4];
+        lane_entries(
+            s, c, p, t, cnt,
+            [&](int i, unsigned e) {
+                ld_record32((e & BND_FLAG ? s.bpv : s.pv) + 2 * (size_t)(e & BND_MASK), pb[i], vb[i]);
+            },
+            [&](int i, int k, unsigned e) {
+                float2 f;
+                div_pair(c, pa, va, pb[i], vb[i], (e & BND_FLAG) != 0u, f.x, f.y);
+                term[q][k] = f;
+            });
+    }
+    __syncwarp();
+    if (act && t == 0) {
+        float acc = 0.f;
+#pragma unroll 4
+        for (int k = 0; k < cnt; ++k) acc = fmaf(term[q][k].x, term[q][k].y, acc);
+        mine = DIV ? div_finish(s, c, p, o, acc) : dens_finish(s, c, p, o, acc, record);
+    }
+    a_partial<BS>(s, mine);
+}
+
+// part B of either loop (k_df_vupdate): lanes 0 to 2 each sum one component
+template <int BS, int DIV, int DECIDE>
+__global__ void __launch_bounds__(BS) k_df_b_lanes(DevScene s, SolverConst c, int parts, double goal_abs, double goal_rel,
+                                                   int min_it, int max_it, cudaGraphConditionalHandle h,
+                                                   int use_handle) {
+    int bid = blockIdx.x;
+    if (DECIDE && parts && bid-- == 0) {
+        b_decide<BS, DIV>(s, c, parts, goal_abs, goal_rel, min_it, max_it, h, use_handle);
+        return;
+    }
+    __shared__ float term[BS / LANES][LROWS * 4];
+    const int n = s.st->n_active;
+    const int t = threadIdx.x % LANES, q = threadIdx.x / LANES;
+    const int p = bid * (BS / LANES) + q;
+    int cnt = 0;
+    float dt = 0.f;
+    float4 va;
+    const bool act = p < n && scene_active(s, s.pv[2 * p]);
+    if (act) {
+        dt = dt_of(s, s.pv[2 * p]);
+        va = s.pv[2 * p + 1];
+        const float4 pa = s.pk[p];
+        cnt = s.ncount[p];
+        float4 pb[4];
+        lane_entries(
+            s, c, p, t, cnt,
+            [&](int i, unsigned e) {
+                const unsigned j = e & BND_MASK;
+                pb[i] = __ldg(e & BND_FLAG ? s.bpv + 2 * (size_t)j : s.pk + j);
+            },
+            [&](int i, int k, unsigned e) {
+                float4 f;
+                v_pair(c, pa, pb[i], (e & BND_FLAG) != 0u, f);
+                *reinterpret_cast<float4*>(&term[q][4 * k]) = f;
+            });
+    }
+    __syncwarp();
+    float d = 0.f;
+    if (act && t < 3) {
+#pragma unroll 4
+        for (int k = 0; k < cnt; ++k) d = fmaf(term[q][4 * k + t], term[q][4 * k + 3], d);
+    }
+    const float dy = __shfl_down_sync(0xffffffffu, d, 1), dz = __shfl_down_sync(0xffffffffu, d, 2);
+    if (act && t == 0) v_finish<DIV>(s, p, va, dt, d, dy, dz);
+}
+
+// non-pressure accelerations and v_adv (k_df_forces); a pair without a force
+// leaves a zero factor
+template <int BS>
+__global__ void __launch_bounds__(BS) k_df_forces_lanes(DevScene s, SolverConst c, int warm) {
+    __shared__ float term[BS / LANES][LROWS * 4];
+    const int n = s.st->n_active;
+    const int t = threadIdx.x % LANES, q = threadIdx.x / LANES;
+    const int p = blockIdx.x * (BS / LANES) + q;
+    int zero = 0, cnt = 0;
+    ForceOwn o;
+    if (p < n) {
+        force_begin(s, c, p, o);
+        cnt = s.ncount[p];
+        float4 pb[4], vb[4];
+        lane_entries(
+            s, c, p, t, cnt,
+            [&](int i, unsigned e) {
+                ld_record32((e & BND_FLAG ? s.bpf : s.prv) + 2 * (size_t)(e & BND_MASK), pb[i], vb[i]);
+            },
+            [&](int i, int k, unsigned e) {
+                float4 f;
+                force_pair(c, o, pb[i], vb[i], (e & BND_FLAG) != 0u, zero, f);
+                *reinterpret_cast<float4*>(&term[q][4 * k]) = f;
+            });
+    }
+    __syncwarp();
+    float a = 0.f;
+    if (p < n && t < 3) {
+        a = c.gravity[t];
+#pragma unroll 4
+        for (int k = 0; k < cnt; ++k) a = fmaf(term[q][4 * k + t], term[q][4 * k + 3], a);
+    }
+    o.ay = __shfl_down_sync(0xffffffffu, a, 1);
+    o.az = __shfl_down_sync(0xffffffffu, a, 2);
+    o.ax = a;
+    if (p < n && t == 0) force_finish(s, c, p, o, warm);
+    if (__syncthreads_or(zero)) {
+        if (zero) atomicAdd(&s.st->zero_dis, zero);
+    }
+}
+
 // FP64 max |v| and the CFL step dt = clamp(cfl * d / vmax, dt_min, dt_max).
 // Each thread takes CFL_ITEMS velocities and the maximum is taken over the
 // squared speeds, with one square root at the end: sqrt is correctly rounded
@@ -489,13 +654,28 @@ void launch_step_begin(const DevScene& s, cudaStream_t st) { k_step_begin<<<1, 1
 void launch_call_begin(const DevScene& s, cudaStream_t st) { k_call_begin<<<1, 1, 0, st>>>(s); }
 void launch_df_loop_reset(const DevScene& s, int which, cudaStream_t st) { k_loop_reset<<<1, 1, 0, st>>>(s, which); }
 
+// the kernels with four threads per particle: 64 or 128 threads (their rows of
+// factors fit the default shared memory)
+#define DISPATCH_LANES(bs, CALL)                        \
+    if (bs == 64) { constexpr int B = 64; CALL; }       \
+    else { constexpr int B = 128; CALL; }
+
 void launch_df_forces(const DevScene& s, const SolverConst& c, int n_max, int warm, cudaStream_t st, int bs) {
-    DISPATCH_BS(bs, (k_df_forces<B><<<nblk(n_max, B), B, 0, st>>>(s, c, warm)));
+    if (c.lanes_a > 1) {
+        DISPATCH_LANES(bs, (k_df_forces_lanes<B><<<nblk(n_max, B / LANES), B, 0, st>>>(s, c, warm)));
+    } else {
+        DISPATCH_BS(bs, (k_df_forces<B><<<nblk(n_max, B), B, 0, st>>>(s, c, warm)));
+    }
 }
 void launch_df_dens_a(const DevScene& s, const SolverConst& c, int n_max, int record, cudaStream_t st, int bs) {
-    DISPATCH_BS(bs, (k_df_dens_a<B><<<nblk(n_max, B), B, 0, st>>>(s, c, record)));
+    if (c.lanes_a > 1) {
+        DISPATCH_LANES(bs, (k_df_a_lanes<B, 0><<<nblk(n_max, B / LANES), B, 0, st>>>(s, c, record)));
+    } else {
+        DISPATCH_BS(bs, (k_df_dens_a<B><<<nblk(n_max, B), B, 0, st>>>(s, c, record)));
+    }
 }
 int df_a_blocks(const SolverConst& c, int n_max, int bs) {
+    if (c.lanes_a > 1) return nblk(n_max, (bs == 64 ? 64 : 128) / LANES);
     return nblk(n_max, bs == 64 || bs == 256 ? bs : 128);
 }
 template <int DIV, int DECIDE>
@@ -505,8 +685,13 @@ static void launch_df_b(const DevScene& s, const SolverConst& c, int n_max, int 
     const cudaGraphConditionalHandle h = (cudaGraphConditionalHandle)cond_handle;
     if (s.nscenes > 1) parts = 0;  // a batch decides per scene
     const int extra = DECIDE && parts ? 1 : 0;
-    DISPATCH_BS(bs, (k_df_vupdate<B, DIV, DECIDE><<<nblk(n_max, B) + extra, B, 0, st>>>(
-                        s, c, parts, goal_abs, goal_rel, min_it, max_it, h, use_handle)));
+    if (c.lanes_b > 1) {
+        DISPATCH_LANES(bs, (k_df_b_lanes<B, DIV, DECIDE><<<nblk(n_max, B / LANES) + extra, B, 0, st>>>(
+                               s, c, parts, goal_abs, goal_rel, min_it, max_it, h, use_handle)));
+    } else {
+        DISPATCH_BS(bs, (k_df_vupdate<B, DIV, DECIDE><<<nblk(n_max, B) + extra, B, 0, st>>>(
+                            s, c, parts, goal_abs, goal_rel, min_it, max_it, h, use_handle)));
+    }
 }
 void launch_df_dens_b(const DevScene& s, const SolverConst& c, int n_max, int parts, double goal, int min_it, int max_it,
                       unsigned long long cond_handle, int use_handle, cudaStream_t st, int bs) {
@@ -516,7 +701,11 @@ void launch_df_warm_correction(const DevScene& s, const SolverConst& c, int n_ma
     launch_df_b<0, 0>(s, c, n_max, 0, 0.0, 0.0, 0, 0, 0ull, 0, st, bs);
 }
 void launch_df_div_a(const DevScene& s, const SolverConst& c, int n_max, cudaStream_t st, int bs) {
-    DISPATCH_BS(bs, (k_df_div_a<B><<<nblk(n_max, B), B, 0, st>>>(s, c)));
+    if (c.lanes_a > 1) {
+        DISPATCH_LANES(bs, (k_df_a_lanes<B, 1><<<nblk(n_max, B / LANES), B, 0, st>>>(s, c, 0)));
+    } else {
+        DISPATCH_BS(bs, (k_df_div_a<B><<<nblk(n_max, B), B, 0, st>>>(s, c)));
+    }
 }
 void launch_df_div_b(const DevScene& s, const SolverConst& c, int n_max, int parts, double goal_abs, double goal_rel,
                      int min_it, int max_it, unsigned long long cond_handle, int use_handle, cudaStream_t st, int bs) {
@@ -532,8 +721,19 @@ static void each_sweep_kernel_bs(F f) {
     f((const void*)k_df_vupdate<B, 0, 0>);
     f((const void*)k_df_vupdate<B, 1, 1>);
 }
+template <int B, class F>
+static void each_lane_kernel_bs(F f) {
+    f((const void*)k_df_forces_lanes<B>);
+    f((const void*)k_df_a_lanes<B, 0>);
+    f((const void*)k_df_a_lanes<B, 1>);
+    f((const void*)k_df_b_lanes<B, 0, 1>);
+    f((const void*)k_df_b_lanes<B, 0, 0>);
+    f((const void*)k_df_b_lanes<B, 1, 1>);
+}
 template <class F>
 static void each_sweep_kernel(F f) {
+    each_lane_kernel_bs<64>(f);
+    each_lane_kernel_bs<128>(f);
     each_sweep_kernel_bs<64>(f);
     each_sweep_kernel_bs<128>(f);
     each_sweep_kernel_bs<256>(f);

@@ -130,6 +130,7 @@ struct sphgpu_scene {
     int l2pol = 1;
     // the list build (SolverConst::build): -1 by size, else 0 or 1 (debug knob "build")
     int build = -1;
+    int sweep_lanes = 0;  // SolverConst::lanes_a, lanes_b: 0 by size, 1 or 4 (debug knob "sweep_lanes")
     int fuse_div = 1;  // DFSPH: the list build performs the divergence loop's first sweep A
     int fuse_ws = 1;   // warm start: features and inference in one kernel
     // set while a step that is not its call's last is enqueued: the step's
@@ -259,6 +260,9 @@ GridGeom make_grid(const SphParams& P) {
 // - / 114 (thread 85); lists only 1 k 44 / 10, 64 k 54 / 37; WCSPH (4 threads
 // per particle) 27 k 34 / 31, 64 k 55 / 51
 constexpr int WARP_BUILD_MAX = 65536;
+// Capacities up to which the DFSPH sweeps run four threads per particle
+// (forces and the A sweeps; the B sweeps); both sides measured in sph_dfsph.cu
+constexpr int LANES_A_MAX = 24000, LANES_B_MAX = 12000;
 void fill_solver_const(sphgpu_scene* h) {
     const SphParams& P = h->P;
     SolverConst& c = h->c;
@@ -299,6 +303,9 @@ void fill_solver_const(sphgpu_scene* h) {
     c.stride = h->stride;
     c.l2pol = h->l2pol;
     c.lanes = h->wc_lanes ? h->wc_lanes : (h->cap <= (1 << 18) ? 4 : 1);
+    const bool lanes_ok = h->ncap <= 48;  // a particle's factors fit its shared-memory row
+    c.lanes_a = lanes_ok && (h->sweep_lanes ? h->sweep_lanes == 4 : h->cap <= LANES_A_MAX) ? 4 : 1;
+    c.lanes_b = lanes_ok && (h->sweep_lanes ? h->sweep_lanes == 4 : h->cap <= LANES_B_MAX) ? 4 : 1;
     c.ws_scale = P.ws_scale;
     // IISph: per-pair h = (d + d)/2 = d (SphBase.h:855-915 with one diameter)
     {
@@ -2918,6 +2925,7 @@ int sphgpu_get_solid_force(sphgpu_t h, int solid_id, double force[3], double tor
 //   carveout_sweeps/_build preferred L1/shared split of the sweeps / list build
 //   l2_policy              L2 eviction priorities of the sweeps' list and record loads
 //   fuse_div               DFSPH: the list build runs the divergence loop's first sweep A
+//   sweep_lanes            threads per particle of the DFSPH sweeps (0 by size, 1, 4)
 //   build                  list build (-1 by size, 0 a thread per particle, 1 a warp for a few)
 //   fuse_ws                warm start: feature gather and network in one kernel
 //   speculative_host_step  sphgpu_step_host runs part 1 while checking its inputs
@@ -2928,6 +2936,13 @@ int sphgpu_debug_set(sphgpu_t h, const char* key, int value) {
     if (k == "record_kappa_sum") { h->record_ksum = value; invalidate_graphs(h); return 0; }
     if (k == "use_graphs") { h->use_graphs = value != 0; return 0; }
     if (k == "fuse_div") { h->fuse_div = value != 0; invalidate_graphs(h); return 0; }
+    if (k == "sweep_lanes") {
+        if (value != 0 && value != 1 && value != 4) return SPHGPU_EINVAL;
+        h->sweep_lanes = value;
+        fill_solver_const(h);
+        invalidate_graphs(h);
+        return 0;
+    }
     if (k == "build") {
         h->build = value;
         fill_solver_const(h);

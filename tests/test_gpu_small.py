@@ -79,3 +79,31 @@ def test_warp_list_build_in_a_batch():
         out.append({"pos": b.get("position"), "vel": b.get("velocity"), "rho": b.get("density")})
         b.close()
     _same(*out)
+
+
+# rows of one entry to full rows, groups of four and their remainders, walls;
+# over the cap; both block sizes
+@pytest.mark.parametrize("kind,counts,kw", [
+    ("block", (1, 1, 1), {}),
+    ("block", (2, 3, 1), {}),
+    ("block", (13, 11, 7), {}),
+    ("block", (26, 31, 29), {}),
+    ("pile", (11, 12, 9), {}),
+    ("block", (9, 9, 9), dict(max_neighbours=10)),
+])
+def test_four_thread_sweeps_are_the_one_thread_sweeps(kind, counts, kw):
+    sc = _scene(kind, counts)
+    steps = 1 if kind == "pile" else 2
+    _same(_run(sc, "dfsph", "sweep_lanes", 1, steps, **kw), _run(sc, "dfsph", "sweep_lanes", 4, steps, **kw))
+
+
+def test_four_thread_sweeps_in_a_batch():
+    scs = [_scene("block", c, seed=k) for k, c in enumerate([(9, 7, 8), (4, 4, 4), (15, 9, 11)])]
+    out = []
+    for value in (1, 4):
+        b = batch_to_gpu(scs, **DF)
+        b.debug_set("sweep_lanes", value)
+        b.step("dfsph", 2)
+        out.append({"pos": b.get("position"), "vel": b.get("velocity"), "rho": b.get("density")})
+        b.close()
+    _same(*out)
