@@ -328,6 +328,10 @@ __global__ void __launch_bounds__(128) k_build_wc_lanes(DevScene s, GridGeom g, 
         float pr = c.wc_B * (powf(density / rho0, c.wc_gamma) - 1.f);
         if (pr < 0.f) pr = 0.f;
         s.kr[p] = pr;
+        // the force pass's record
+        const float4 v = s.vel[p];
+        s.prv[2 * p] = make_float4(pa.x, pa.y, pa.z, density);
+        s.prv[2 * p + 1] = make_float4(v.x, v.y, v.z, pr / (density * density));
     }
     __shared__ int sh[BS / 32];
     const bool lead = act && l == 0;

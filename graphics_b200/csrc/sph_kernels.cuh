@@ -70,7 +70,8 @@ struct DevScene {
     float4* pk;         // (x, y, z, kappa/rho) -- the record the B sweeps gather
     float4* prv;        // 2 per particle: {(x, y, z, rho), velocity} -- the record the
                         // DFSPH force kernel gathers (position and rho from the list
-                        // build, velocity from the reorder / divergence sweep)
+                        // build, velocity from the reorder / divergence sweep); WCSPH:
+                        // w of the velocity p/rho^2 (all from the list build)
     float4* bpv;        // 2 per boundary particle: {(x,y,z,volume), velocity}
     float4* bpf;        // the record the DFSPH force kernel gathers for a boundary
                         // particle: {(x,y,z,volume), singleVelocity + velocity}

@@ -169,8 +169,50 @@ __device__ __forceinline__ void wc_finish(const DevScene& s, const WcOwn& o, int
     s.gid_s[p] = s.gid[p];
 }
 
-// one thread per particle, neighbours in list order
-template <bool SURF>
+// One fluid phase without surface terms: a neighbour is one 32-byte record
+// {(x, y, z, rho), (v, p/rho^2)} written by the list build (boundary:
+// {(x, y, z, volume), v}) instead of four gathers, its p/rho^2 divided once
+// per particle instead of once per pair, -W'(r)/r taken from one rsqrt and
+// the viscosity's two divisions joined into one reciprocal (velocities after
+// 20 steps are 5e-6 off FP64 either way).  Terms as wc_pair.  Event-timed,
+// four gathers one after the other / one record, four in flight: 27 k
+// particles (4 threads each) 22.0 / 11.2 us, 512 k (1 thread) 160 / 69.
+struct WcPlain {
+    float4 pa, va;
+    float fma, bm, bterm, visc, bnu, den0, ra, pa_term;
+};
+__device__ __forceinline__ WcPlain wc_plain(const WcOwn& o, const SolverConst& c) {
+    WcPlain w;
+    w.pa = o.pa;
+    w.va = o.va;
+    w.fma = -o.fma;
+    w.bm = -o.rho0;
+    w.bterm = o.pra > 0.f ? o.pa_term * 2.f : 0.f;
+    w.visc = -2.f * o.alpha * c.hs * c.cs;
+    w.bnu = -2.f * c.bvisc * c.hs * c.cs / (o.ra * 2.f);
+    w.den0 = o.den0;
+    w.ra = o.ra;
+    w.pa_term = o.pa_term;
+    return w;
+}
+__device__ __forceinline__ void wc_term(const SolverConst& c, const WcPlain& o, float4 pb, float4 vb, bool bnd,
+                                        float& ax, float& ay, float& az, int& zero) {
+    const float xx = o.pa.x - pb.x, xy = o.pa.y - pb.y, xz = o.pa.z - pb.z;
+    const float len2 = xx * xx + xy * xy + xz * xz;
+    if (len2 == 0.f) { ++zero; return; }
+    const float f = grad_over_r(c.k, len2);
+    const float pro = fminf((o.va.x - vb.x) * xx + (o.va.y - vb.y) * xy + (o.va.z - vb.z) * xz, 0.f);
+    const float den = len2 + o.den0;
+    // pressure and viscosity terms of the pair, times -m_j
+    const float acce = bnd ? f * (o.bm * pb.w) * (o.bterm + o.bnu * pro * __frcp_rn(den))
+                           : f * o.fma * (o.pa_term + vb.w + o.visc * pro * __frcp_rn(den * (o.ra + pb.w)));
+    ax = fmaf(xx, acce, ax);
+    ay = fmaf(xy, acce, ay);
+    az = fmaf(xz, acce, az);
+}
+
+// one thread per particle, neighbours in list order, four records in flight
+template <bool SURF, bool PLAIN>
 __global__ void __launch_bounds__(NT) k_wc_force(DevScene s, SolverConst c) {
     const int n = s.st->n_active;
     const int p = blockIdx.x * NT + threadIdx.x;
@@ -180,7 +222,31 @@ __global__ void __launch_bounds__(NT) k_wc_force(DevScene s, SolverConst c) {
         float ax = c.gravity[0], ay = c.gravity[1], az = c.gravity[2];
         const int cnt = s.ncount[p];
         const size_t stride = (size_t)c.stride;
-        for (int k = 0; k < cnt; ++k) wc_pair<SURF>(s, c, o, p, (unsigned)ell_get(s.nbr, stride, p, k), ax, ay, az, zero);
+        if (PLAIN) {
+            const WcPlain w = wc_plain(o, c);
+            const unsigned long long polL = l2_policy(c.l2pol & 3);  // lists stream through L2
+            const int ng = (cnt + 3) >> 2;
+            int4 nxt = ng ? ell_group_pol(s.nbr, stride, p, 0, polL) : make_int4(0, 0, 0, 0);
+            for (int gi = 0; gi < ng; ++gi) {
+                const int4 cur = nxt;
+                if (gi + 1 < ng) nxt = ell_group_pol(s.nbr, stride, p, gi + 1, polL);
+                const unsigned e[4] = {(unsigned)cur.x, (unsigned)cur.y, (unsigned)cur.z, (unsigned)cur.w};
+                float4 pb[4], vb[4];
+                bool bnd[4];
+#pragma unroll
+                for (int t = 0; t < 4; ++t) {
+                    // entries past the count read the particle's own record
+                    const unsigned u = gi * 4 + t < cnt ? e[t] : (unsigned)p;
+                    bnd[t] = (u & BND_FLAG) != 0u;
+                    ld_record32((bnd[t] ? s.bpv : s.prv) + 2 * (size_t)(u & BND_MASK), pb[t], vb[t]);
+                }
+#pragma unroll
+                for (int t = 0; t < 4; ++t)
+                    if (gi * 4 + t < cnt) wc_term(c, w, pb[t], vb[t], bnd[t], ax, ay, az, zero);
+            }
+        } else {
+            for (int k = 0; k < cnt; ++k) wc_pair<SURF>(s, c, o, p, (unsigned)ell_get(s.nbr, stride, p, k), ax, ay, az, zero);
+        }
         wc_finish(s, o, p, ax, ay, az);
     }
     if (__syncthreads_or(zero)) {
@@ -192,7 +258,7 @@ __global__ void __launch_bounds__(NT) k_wc_force(DevScene s, SolverConst c) {
 // leaves the SMs with too few warps to hide the gathers' latency): lane l
 // takes neighbours l, l + L, ...; the lanes' sums are added in a fixed
 // shuffle order (deterministic), the group's first lane integrates
-template <bool SURF, int L>
+template <bool SURF, bool PLAIN, int L>
 __global__ void __launch_bounds__(NT) k_wc_force_lanes(DevScene s, SolverConst c) {
     const int n = s.st->n_active;
     const int t = blockIdx.x * NT + threadIdx.x;
@@ -205,7 +271,24 @@ __global__ void __launch_bounds__(NT) k_wc_force_lanes(DevScene s, SolverConst c
         if (l == 0) { ax = c.gravity[0]; ay = c.gravity[1]; az = c.gravity[2]; }
         const int cnt = s.ncount[p];
         const size_t stride = (size_t)c.stride;
-        for (int k = l; k < cnt; k += L) wc_pair<SURF>(s, c, o, p, (unsigned)ell_get(s.nbr, stride, p, k), ax, ay, az, zero);
+        if (PLAIN) {
+            const WcPlain w = wc_plain(o, c);
+            for (int k0 = l; k0 < cnt; k0 += 4 * L) {
+                unsigned u[4];
+                float4 pb[4], vb[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    u[i] = k0 + i * L < cnt ? (unsigned)ell_get(s.nbr, stride, p, k0 + i * L) : (unsigned)p;
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    ld_record32((u[i] & BND_FLAG ? s.bpv : s.prv) + 2 * (size_t)(u[i] & BND_MASK), pb[i], vb[i]);
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    if (k0 + i * L < cnt) wc_term(c, w, pb[i], vb[i], (u[i] & BND_FLAG) != 0u, ax, ay, az, zero);
+            }
+        } else {
+            for (int k = l; k < cnt; k += L) wc_pair<SURF>(s, c, o, p, (unsigned)ell_get(s.nbr, stride, p, k), ax, ay, az, zero);
+        }
     }
 #pragma unroll
     for (int off = 1; off < L; off <<= 1) {
@@ -223,12 +306,15 @@ __global__ void __launch_bounds__(NT) k_wc_force_lanes(DevScene s, SolverConst c
 void launch_wc_force(const DevScene& s, const SolverConst& c, int n_max, cudaStream_t st, bool surf, int lanes) {
     if (lanes == 4) {
         const int nb = (int)(((long long)n_max * 4 + NT - 1) / NT);
-        if (surf) k_wc_force_lanes<true, 4><<<nb, NT, 0, st>>>(s, c);
-        else k_wc_force_lanes<false, 4><<<nb, NT, 0, st>>>(s, c);
+        if (surf) k_wc_force_lanes<true, false, 4><<<nb, NT, 0, st>>>(s, c);
+        else if (c.nphase == 1) k_wc_force_lanes<false, true, 4><<<nb, NT, 0, st>>>(s, c);
+        else k_wc_force_lanes<false, false, 4><<<nb, NT, 0, st>>>(s, c);
         return;
     }
-    if (surf) k_wc_force<true><<<(n_max + NT - 1) / NT, NT, 0, st>>>(s, c);
-    else k_wc_force<false><<<(n_max + NT - 1) / NT, NT, 0, st>>>(s, c);
+    const int nb = (n_max + NT - 1) / NT;
+    if (surf) k_wc_force<true, false><<<nb, NT, 0, st>>>(s, c);
+    else if (c.nphase == 1) k_wc_force<false, true><<<nb, NT, 0, st>>>(s, c);
+    else k_wc_force<false, false><<<nb, NT, 0, st>>>(s, c);
 }
 void launch_wc_normal(const DevScene& s, const SolverConst& c, int n_max, cudaStream_t st) {
     k_wc_normal<<<(n_max + NT - 1) / NT, NT, 0, st>>>(s, c);

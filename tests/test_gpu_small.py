@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 
 from graphics_b200.scene import dam_break, rayleigh_taylor
-from graphics_b200.sph import batch_to_gpu, scene_to_gpu
+from graphics_b200.sph import GpuScene, batch_to_gpu, params_for_scene, scene_to_gpu
 
 pytestmark = pytest.mark.gpu
 
@@ -107,3 +107,26 @@ def test_four_thread_sweeps_in_a_batch():
         out.append({"pos": b.get("position"), "vel": b.get("velocity"), "rho": b.get("density")})
         b.close()
     _same(*out)
+
+
+# WCSPH's plain force pass (one record per neighbour) against the general
+# one, which a scene of two fluids takes: here the second is one particle out
+# of reach in the far corner; both thread counts
+@pytest.mark.parametrize("lanes", [1, 4])
+@pytest.mark.parametrize("counts", [(1, 1, 1), (2, 3, 2), (13, 11, 12)])
+def test_wcsph_plain_forces_match_the_general_pass(lanes, counts):
+    sc = _scene("block", counts)
+    acc = []
+    for far in (False, True):
+        g = GpuScene(params_for_scene(sc, **KW["wcsph"], boundary_visc=0.03), sc.n_fluid + 1)
+        g.debug_set("wc_lanes", lanes)
+        g.set_boundary(sc.boundary_pos)
+        g.add_fluid(sc.fluid_pos, sc.fluid_vel, visc_alpha=0.05)
+        if far:
+            corner = np.array([[(k + 2.5) * sc.d for k in counts]], np.float32)
+            g.add_fluid(corner, rho0=2000.0, visc_alpha=0.05)
+        g.step("wcsph", 1)
+        acc.append(g.get("acceleration")[:sc.n_fluid])
+        g.close()
+    # some 50 terms, each a few ulp of the largest, in either pass: 50 * 4 * 2^-24
+    assert np.abs(acc[0] - acc[1]).max() <= 50 * 4 * 2.0 ** -24 * np.abs(acc[0]).max()
