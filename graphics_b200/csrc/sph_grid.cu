@@ -111,7 +111,13 @@ __global__ void __launch_bounds__(NT) k_rank_reorder(DevScene s, int dead_key, i
     s.gid[p] = my;
     if (carry & 1) s.hist[p] = s.hist_s[i];
     if (carry & 2) s.cA[p] = s.cA_s[i];
-    if (carry & 4) s.cB[p] = s.cB_s[i];
+    if (carry & 4) {
+        const float4 b = s.cB_s[i];
+        s.cB[p] = b;
+        // the record of the PCISPH / IISPH_M non-pressure forces
+        s.prv[2 * p] = x;
+        s.prv[2 * p + 1] = make_float4(v.x, v.y, v.z, b.w);
+    }
     if (carry & 8) s.cC[p] = s.cC_s[i];
 }
 

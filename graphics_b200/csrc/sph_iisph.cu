@@ -146,35 +146,43 @@ __global__ void __launch_bounds__(BS) k_iv_forces(DevScene s, SolverConst c) {
         const float den0 = 0.01f * c.hs * c.hs;
         float ax = c.gravity[0], ay = c.gravity[1], az = c.gravity[2];
         const int cnt = s.ncount[p];
-        const size_t stride = (size_t)c.stride;
-        for (int k = 0; k < cnt; ++k) {
-            const unsigned e = (unsigned)ell_get(s.nbr, stride, p, k);
-            const bool bnd = (e & BND_FLAG) != 0u;
-            const unsigned j = e & BND_MASK;
-            const float4 pb = bnd ? s.bpos[j] : s.pos[j];
-            const float4 vb = bnd ? s.bvel[j] : s.vel[j];
-            const float xx = pa.x - pb.x, xy = pa.y - pb.y, xz = pa.z - pb.z;
-            const float len2 = xx * xx + xy * xy + xz * xz;
-            if (len2 == 0.f) { ++zero; continue; }
-            const float pro = (va.x - vb.x) * xx + (va.y - vb.y) * xy + (va.z - vb.z) * xz;
-            float t;
-            if (bnd || phase_of(pb) == ph) {
-                const float vg = bnd ? pb.w / s.bivs[j].x : Va / s.ivs[j].x;
-                const float f = grad_over_r(c.kd, len2);
-                t = f * 10.f * (bnd ? kvb : kvf) * vg * pro / (len2 + 1e-6f);
-            } else {
-                if (!(pro < 0.f)) continue;
-                const int phb = phase_of(pb);
-                const float fmb = Va * c.rho0_ph[phb];
-                const float al = (alpha + c.alpha_ph[phb]) / 2.f;
-                const float nu = 2.f * al * c.hs * c.cs / (rhoa + s.ivs[j].w);
-                const float pi = -nu * pro / (len2 + den0);
-                t = grad_over_r(c.k, len2) * (-(ma + fmb) / 2.f * pi);
-            }
-            ax = fmaf(xx, t, ax);
-            ay = fmaf(xy, t, ay);
-            az = fmaf(xz, t, az);
-        }
+        float4 pbs[4], vbs[4];
+        float gs[4];
+        walk4(
+            s.nbr, (size_t)c.stride, p, cnt, (unsigned)p, l2_policy(c.l2pol & 3),
+            [&](int q, unsigned u) {
+                const bool b = (u & BND_FLAG) != 0u;
+                const unsigned j = u & BND_MASK;
+                pbs[q] = __ldg((b ? s.bpos : s.pos) + j);
+                vbs[q] = __ldg((b ? s.bvel : s.vel) + j);
+                gs[q] = __ldg(&(b ? s.bivs : s.ivs)[j].x);
+            },
+            [&](int q, unsigned u) {
+                const bool bnd = (u & BND_FLAG) != 0u;
+                const unsigned j = u & BND_MASK;
+                const float4 pb = pbs[q], vb = vbs[q];
+                const float xx = pa.x - pb.x, xy = pa.y - pb.y, xz = pa.z - pb.z;
+                const float len2 = xx * xx + xy * xy + xz * xz;
+                if (len2 == 0.f) { ++zero; return; }
+                const float pro = (va.x - vb.x) * xx + (va.y - vb.y) * xy + (va.z - vb.z) * xz;
+                float t;
+                if (bnd || phase_of(pb) == ph) {
+                    const float vg = (bnd ? pb.w : Va) / gs[q];
+                    const float f = grad_over_r(c.kd, len2);
+                    t = f * 10.f * (bnd ? kvb : kvf) * vg * pro / (len2 + 1e-6f);
+                } else {
+                    if (!(pro < 0.f)) return;
+                    const int phb = phase_of(pb);
+                    const float fmb = Va * c.rho0_ph[phb];
+                    const float al = (alpha + c.alpha_ph[phb]) / 2.f;
+                    const float nu = 2.f * al * c.hs * c.cs / (rhoa + s.ivs[j].w);
+                    const float pi = -nu * pro / (len2 + den0);
+                    t = grad_over_r(c.k, len2) * (-(ma + fmb) / 2.f * pi);
+                }
+                ax = fmaf(xx, t, ax);
+                ay = fmaf(xy, t, ay);
+                az = fmaf(xz, t, az);
+            });
         s.acc[p] = make_float4(ax, ay, az, 0.f);
         const float4 ca = s.cA[p], cc = s.cC[p];
         s.pv[2 * p + 1] = make_float4(ca.x, ca.y, ca.z, 0.f);
@@ -274,15 +282,17 @@ __global__ void __launch_bounds__(BS) k_iv_boundary_sweep(DevScene s, SolverCons
     const int cnt = s.bncount[p];
     const size_t bstride = (size_t)s.bstride;
     float acc = 0.f;
-    for (int k = 0; k < cnt; ++k) {
-        const int j = s.bnbr[ell_index(bstride, p, k)];
-        float4 pb, vb;
-        ld_record32(s.pv + 2 * (size_t)j, pb, vb);
-        const float xx = pa.x - pb.x, xy = pa.y - pb.y, xz = pa.z - pb.z;
-        const float f = grad_over_r(c.kd, xx * xx + xy * xy + xz * xz);
-        const float dot = xx * (vb0.x - vb.x) + xy * (vb0.y - vb.y) + xz * (vb0.z - vb.z);
-        acc = fmaf(dot * f, c.iv_V, acc);
-    }
+    float4 pbs[4], vbs[4];
+    walk4(
+        s.bnbr, bstride, p, cnt, 0u, l2_policy(c.l2pol & 3),
+        [&](int t, unsigned u) { ld_record32(s.pv + 2 * (size_t)u, pbs[t], vbs[t]); },
+        [&](int t, unsigned) {
+            const float4 pb = pbs[t], vb = vbs[t];
+            const float xx = pa.x - pb.x, xy = pa.y - pb.y, xz = pa.z - pb.z;
+            const float f = grad_over_r(c.kd, xx * xx + xy * xy + xz * xz);
+            const float dot = xx * (vb0.x - vb.x) + xy * (vb0.y - vb.y) + xz * (vb0.z - vb.z);
+            acc = fmaf(dot * f, c.iv_V, acc);
+        });
     float4 o = s.bivo[p];
     float kap;
     if (DIV) {
@@ -307,7 +317,7 @@ __global__ void __launch_bounds__(BS) k_iv_boundary_sweep(DevScene s, SolverCons
 // change or divergence, clamp, stiffness kappa (pk.w = kappa/gamma), FP64
 // sum of the error term: (V_adv - V)/V (constant volume) or the divergence.
 template <int BS, int DIV>
-__global__ void __launch_bounds__(BS) k_iv_sweep_a(DevScene s, SolverConst c, int phase) {
+__global__ void __launch_bounds__(BS, 1024 / BS) k_iv_sweep_a(DevScene s, SolverConst c, int phase) {
     const int n = s.st->n_active;
     const int p = blockIdx.x * BS + threadIdx.x;
     double mine = 0.0;

@@ -71,7 +71,9 @@ struct DevScene {
     float4* prv;        // 2 per particle: {(x, y, z, rho), velocity} -- the record the
                         // DFSPH force kernel gathers (position and rho from the list
                         // build, velocity from the reorder / divergence sweep); WCSPH:
-                        // w of the velocity p/rho^2 (all from the list build)
+                        // w of the velocity p/rho^2 (all from the list build); the
+                        // non-pressure forces of PCISPH and IISPH_M: {position, (velocity,
+                        // density of the previous step)} from the reorder
     float4* bpv;        // 2 per boundary particle: {(x,y,z,volume), velocity}
     float4* bpf;        // the record the DFSPH force kernel gathers for a boundary
                         // particle: {(x,y,z,volume), singleVelocity + velocity}
@@ -237,6 +239,30 @@ __device__ __forceinline__ float div_term(const SolverConst& c, float4 pa, float
     float t, m;
     div_pair(c, pa, va, pb, vb, bnd, t, m);
     return fmaf(t, m, acc);
+}
+
+// Walks an ELL list of cnt entries by one thread, four at a time: the next
+// group's load is issued before ld(t, entry), t < 4, issues the current
+// one's gathers (entries past the count: `self`), then use(t, entry) takes
+// the entries of the list in order.
+template <class Ld, class Use>
+__device__ __forceinline__ void walk4(const int* list, size_t stride, int p, int cnt, unsigned self,
+                                      unsigned long long pol, Ld&& ld, Use&& use) {
+    const int ng = (cnt + 3) >> 2;
+    int4 nxt = ng ? ell_group_pol(list, stride, p, 0, pol) : make_int4(0, 0, 0, 0);
+    for (int gi = 0; gi < ng; ++gi) {
+        const int4 cur = nxt;
+        if (gi + 1 < ng) nxt = ell_group_pol(list, stride, p, gi + 1, pol);
+        unsigned e[4] = {(unsigned)cur.x, (unsigned)cur.y, (unsigned)cur.z, (unsigned)cur.w};
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            if (gi * 4 + t >= cnt) e[t] = self;
+            ld(t, e[t]);
+        }
+#pragma unroll
+        for (int t = 0; t < 4; ++t)
+            if (gi * 4 + t < cnt) use(t, e[t]);
+    }
 }
 
 // ---- neighbour search (sph_grid.cu) ----

@@ -108,43 +108,45 @@ __global__ void __launch_bounds__(NT) k_pci_force_except(DevScene s, SolverConst
         const float hscs = c.hs * c.cs;
         float ax = c.gravity[0], ay = c.gravity[1], az = c.gravity[2];
         const int cnt = s.ncount[p];
-        const size_t stride = (size_t)c.stride;
-        for (int k = 0; k < cnt; ++k) {
-            bool bnd;
-            unsigned j;
-            nbr_fetch(s, (unsigned)ell_get(s.nbr, stride, p, k), bnd, j);
-            const float4 pb = bnd ? s.bpos[j] : s.pos[j];
-            const float4 vb = bnd ? s.bvel[j] : s.vel[j];
-            const float xx = pa.x - pb.x, xy = pa.y - pb.y, xz = pa.z - pb.z;
-            const float len2 = xx * xx + xy * xy + xz * xz;
-            if (len2 == 0.f) { ++zero; continue; }
-            const float pro = (va.x - vb.x) * xx + (va.y - vb.y) * xy + (va.z - vb.z) * xz;
-            if (!(pro < 0.f)) continue;
-            const float f = grad_over_r(c.k, len2);
-            float acce;
-            if (bnd) {
-                // PciSph.cpp:218-224
-                const float nu = 2.f * c.bvisc * hscs / (ra * 2.f);
-                const float pi = -nu * pro / (len2 + den0);
-                acce = f * (-rho0 * pb.w * pi);
-            } else {
-                const float rb = s.cB[j].w;
-                const int phb = phase_of(pb);
-                if (phb == ph) {  // PciSph.cpp:178-184
-                    const float nu = 2.f * alpha * hscs / (ra + rb);
+        float4 pbs[4], vbs[4];
+        walk4(
+            s.nbr, (size_t)c.stride, p, cnt, (unsigned)p, l2_policy(c.l2pol & 3),
+            [&](int t, unsigned u) {
+                ld_record32((u & BND_FLAG ? s.bpv : s.prv) + 2 * (size_t)(u & BND_MASK), pbs[t], vbs[t]);
+            },
+            [&](int t, unsigned u) {
+                const bool bnd = (u & BND_FLAG) != 0u;
+                const float4 pb = pbs[t], vb = vbs[t];
+                const float xx = pa.x - pb.x, xy = pa.y - pb.y, xz = pa.z - pb.z;
+                const float len2 = xx * xx + xy * xy + xz * xz;
+                if (len2 == 0.f) { ++zero; return; }
+                const float pro = (va.x - vb.x) * xx + (va.y - vb.y) * xy + (va.z - vb.z) * xz;
+                if (!(pro < 0.f)) return;
+                const float f = grad_over_r(c.k, len2);
+                float acce;
+                if (bnd) {
+                    // PciSph.cpp:218-224
+                    const float nu = 2.f * c.bvisc * hscs / (ra * 2.f);
                     const float pi = -nu * pro / (len2 + den0);
-                    acce = f * (-fm0 * pi);
-                } else {          // PciSph.cpp:198-204
-                    const float al = (alpha + c.alpha_ph[phb]) / 2.f;
-                    const float nu = 2.f * al * hscs / (ra + rb);
-                    const float pi = -nu * pro / (len2 + den0);
-                    acce = f * (-(fm0 + c.fm_ph[phb]) / 2.f * pi);
+                    acce = f * (-rho0 * pb.w * pi);
+                } else {
+                    const float rb = vb.w;
+                    const int phb = phase_of(pb);
+                    if (phb == ph) {  // PciSph.cpp:178-184
+                        const float nu = 2.f * alpha * hscs / (ra + rb);
+                        const float pi = -nu * pro / (len2 + den0);
+                        acce = f * (-fm0 * pi);
+                    } else {          // PciSph.cpp:198-204
+                        const float al = (alpha + c.alpha_ph[phb]) / 2.f;
+                        const float nu = 2.f * al * hscs / (ra + rb);
+                        const float pi = -nu * pro / (len2 + den0);
+                        acce = f * (-(fm0 + c.fm_ph[phb]) / 2.f * pi);
+                    }
                 }
-            }
-            ax = fmaf(xx, acce, ax);
-            ay = fmaf(xy, acce, ay);
-            az = fmaf(xz, acce, az);
-        }
+                ax = fmaf(xx, acce, ax);
+                ay = fmaf(xy, acce, ay);
+                az = fmaf(xz, acce, az);
+            });
         s.acc[p] = make_float4(ax, ay, az, 0.f);
         s.ap[p] = make_float4(0.f, 0.f, 0.f, 0.f);
         s.kr[p] = 0.f;
@@ -350,38 +352,40 @@ __global__ void __launch_bounds__(NT) k_ii_force_except(DevScene s, SolverConst 
         const float visc = 10.f * c.nu;
         float ax = c.gravity[0], ay = c.gravity[1], az = c.gravity[2];
         const int cnt = s.ncount[p];
-        const size_t stride = (size_t)c.stride;
-        for (int k = 0; k < cnt; ++k) {
-            bool bnd;
-            unsigned j;
-            nbr_fetch(s, (unsigned)ell_get(s.nbr, stride, p, k), bnd, j);
-            const float4 pb = bnd ? s.bpos[j] : s.pos[j];
-            const float4 vb = bnd ? s.bvel[j] : s.vel[j];
-            const float xx = pa.x - pb.x, xy = pa.y - pb.y, xz = pa.z - pb.z;
-            const float len2 = xx * xx + xy * xy + xz * xz;
-            if (len2 == 0.f) { ++zero; continue; }
-            const float pro = (va.x - vb.x) * xx + (va.y - vb.y) * xy + (va.z - vb.z) * xz;
-            const float f = grad_over_r(c.k, len2);
-            float t;
-            if (bnd) {
-                t = f * pro / (len2 + den0) * (rho0 * pb.w) / ra * visc;
-            } else {
-                const int phb = phase_of(pb);
-                const float rb = s.cB[j].w;
-                if (phb == ph) {
-                    t = f * pro / (len2 + den0) * fm0 / rb * visc;
+        float4 pbs[4], vbs[4];
+        walk4(
+            s.nbr, (size_t)c.stride, p, cnt, (unsigned)p, l2_policy(c.l2pol & 3),
+            [&](int q, unsigned u) {
+                ld_record32((u & BND_FLAG ? s.bpv : s.prv) + 2 * (size_t)(u & BND_MASK), pbs[q], vbs[q]);
+            },
+            [&](int q, unsigned u) {
+                const bool bnd = (u & BND_FLAG) != 0u;
+                const float4 pb = pbs[q], vb = vbs[q];
+                const float xx = pa.x - pb.x, xy = pa.y - pb.y, xz = pa.z - pb.z;
+                const float len2 = xx * xx + xy * xy + xz * xz;
+                if (len2 == 0.f) { ++zero; return; }
+                const float pro = (va.x - vb.x) * xx + (va.y - vb.y) * xy + (va.z - vb.z) * xz;
+                const float f = grad_over_r(c.k, len2);
+                float t;
+                if (bnd) {
+                    t = f * pro / (len2 + den0) * (rho0 * pb.w) / ra * visc;
                 } else {
-                    if (!(pro < 0.f)) continue;
-                    const float al = (alpha + c.alpha_ph[phb]) / 2.f;
-                    const float nu = 2.f * al * c.hs * c.cs / (ra + rb);
-                    const float pi = -nu * pro / (len2 + den0);
-                    t = f * (-(fm0 + c.fm_ph[phb]) / 2.f * pi);
+                    const int phb = phase_of(pb);
+                    const float rb = vb.w;
+                    if (phb == ph) {
+                        t = f * pro / (len2 + den0) * fm0 / rb * visc;
+                    } else {
+                        if (!(pro < 0.f)) return;
+                        const float al = (alpha + c.alpha_ph[phb]) / 2.f;
+                        const float nu = 2.f * al * c.hs * c.cs / (ra + rb);
+                        const float pi = -nu * pro / (len2 + den0);
+                        t = f * (-(fm0 + c.fm_ph[phb]) / 2.f * pi);
+                    }
                 }
-            }
-            ax = fmaf(xx, t, ax);
-            ay = fmaf(xy, t, ay);
-            az = fmaf(xz, t, az);
-        }
+                ax = fmaf(xx, t, ax);
+                ay = fmaf(xy, t, ay);
+                az = fmaf(xz, t, az);
+            });
         s.acc[p] = make_float4(ax, ay, az, 0.f);
         s.kr[p] = 0.f;
     }
@@ -401,7 +405,7 @@ __global__ void k_ii_phase_begin(DevScene s) {
 
 // rho = m_k (W(0) + sum_f W) + sum_b rho0_k V_b W; d_ii = -dt^2 sum m_j/rho^2 gradW;
 // v_adv = v + a_adv dt (IISph_M.cpp:94-136)
-__global__ void __launch_bounds__(NT) k_ii_density(DevScene s, SolverConst c, int phase) {
+__global__ void __launch_bounds__(NT, 8) k_ii_density(DevScene s, SolverConst c, int phase) {
     const int n = s.st->n_active;
     const int p = blockIdx.x * NT + threadIdx.x;
     int mine = 0;
@@ -414,23 +418,24 @@ __global__ void __launch_bounds__(NT) k_ii_density(DevScene s, SolverConst c, in
             float density = ker_W(c.k, 0.f) * fm0;
             float gx = 0.f, gy = 0.f, gz = 0.f;
             const int cnt = s.ncount[p];
-            const size_t stride = (size_t)c.stride;
-            for (int k = 0; k < cnt; ++k) {
-                bool bnd;
-                unsigned j;
-                nbr_fetch(s, (unsigned)ell_get(s.nbr, stride, p, k), bnd, j);
-                const float4 pb = bnd ? s.bpos[j] : s.pos[j];
-                const float xx = pa.x - pb.x, xy = pa.y - pb.y, xz = pa.z - pb.z;
-                const float len2 = xx * xx + xy * xy + xz * xz;
-                float w, f;
-                kernel_pair(c.k, len2, w, f);
-                const float m = bnd ? rho0 * pb.w : fm0;
-                density = fmaf(m, w, density);
-                const float fm = f * m;
-                gx = fmaf(xx, fm, gx);
-                gy = fmaf(xy, fm, gy);
-                gz = fmaf(xz, fm, gz);
-            }
+            float4 pbs[4];
+            walk4(
+                s.nbr, (size_t)c.stride, p, cnt, (unsigned)p, l2_policy(c.l2pol & 3),
+                [&](int t, unsigned u) { pbs[t] = __ldg((u & BND_FLAG ? s.bpos : s.pos) + (u & BND_MASK)); },
+                [&](int t, unsigned u) {
+                    const bool bnd = (u & BND_FLAG) != 0u;
+                    const float4 pb = pbs[t];
+                    const float xx = pa.x - pb.x, xy = pa.y - pb.y, xz = pa.z - pb.z;
+                    const float len2 = xx * xx + xy * xy + xz * xz;
+                    float w, f;
+                    kernel_pair(c.k, len2, w, f);
+                    const float m = bnd ? rho0 * pb.w : fm0;
+                    density = fmaf(m, w, density);
+                    const float fm = f * m;
+                    gx = fmaf(xx, fm, gx);
+                    gy = fmaf(xy, fm, gy);
+                    gz = fmaf(xz, fm, gz);
+                });
             const float q = -(dt * dt) / (density * density);
             s.cB[p] = make_float4(gx * q, gy * q, gz * q, density);
             s.rho[p] = density;
@@ -448,7 +453,7 @@ __global__ void __launch_bounds__(NT) k_ii_density(DevScene s, SolverConst c, in
 }
 
 // a_ii, rho_adv, p_l = p/2 (IISph_M.cpp:243-278)
-__global__ void __launch_bounds__(NT) k_ii_aii(DevScene s, SolverConst c, int phase) {
+__global__ void __launch_bounds__(NT, 8) k_ii_aii(DevScene s, SolverConst c, int phase) {
     const int n = s.st->n_active;
     const int p = blockIdx.x * NT + threadIdx.x;
     if (p >= n) return;
@@ -469,26 +474,32 @@ __global__ void __launch_bounds__(NT) k_ii_aii(DevScene s, SolverConst c, int ph
     const float qd = fm0 * dt * dt / (ra * ra);
     float tv1 = 0.f, tv2 = 0.f;
     const int cnt = s.ncount[p];
-    const size_t stride = (size_t)c.stride;
-    for (int k = 0; k < cnt; ++k) {
-        bool bnd;
-        unsigned j;
-        nbr_fetch(s, (unsigned)ell_get(s.nbr, stride, p, k), bnd, j);
-        const float4 pb = bnd ? s.bpos[j] : s.pos[j];
-        const float xx = pa.x - pb.x, xy = pa.y - pb.y, xz = pa.z - pb.z;
-        const float f = grad_over_r(c.k, xx * xx + xy * xy + xz * xz);
-        const float g0 = xx * f, g1 = xy * f, g2 = xz * f;
-        if (bnd) {
-            const float4 vb = s.bvel[j];
-            const float m = rho0 * pb.w;
-            tv1 += (g0 * (va.x - vb.x) + g1 * (va.y - vb.y) + g2 * (va.z - vb.z)) * m * dt;
-            tv2 += (da.x * g0 + da.y * g1 + da.z * g2) * m;
-        } else {
-            const float4 wb = s.cA[j];
-            tv1 += (g0 * (wa.x - wb.x) + g1 * (wa.y - wb.y) + g2 * (wa.z - wb.z)) * fm0 * dt;
-            tv2 += ((da.x - g0 * qd) * g0 + (da.y - g1 * qd) * g1 + (da.z - g2 * qd) * g2) * fm0;
-        }
-    }
+    float4 pbs[4], wbs[4];
+    walk4(
+        s.nbr, (size_t)c.stride, p, cnt, (unsigned)p, l2_policy(c.l2pol & 3),
+        [&](int t, unsigned u) {
+            const unsigned j = u & BND_MASK;
+            pbs[t] = __ldg((u & BND_FLAG ? s.bpos : s.pos) + j);
+            // of cA only v_adv is used (this kernel writes the w)
+            wbs[t] = (u & BND_FLAG ? s.bvel : s.cA)[j];
+        },
+        [&](int t, unsigned u) {
+            const bool bnd = (u & BND_FLAG) != 0u;
+            const float4 pb = pbs[t];
+            const float xx = pa.x - pb.x, xy = pa.y - pb.y, xz = pa.z - pb.z;
+            const float f = grad_over_r(c.k, xx * xx + xy * xy + xz * xz);
+            const float g0 = xx * f, g1 = xy * f, g2 = xz * f;
+            if (bnd) {
+                const float4 vb = wbs[t];
+                const float m = rho0 * pb.w;
+                tv1 += (g0 * (va.x - vb.x) + g1 * (va.y - vb.y) + g2 * (va.z - vb.z)) * m * dt;
+                tv2 += (da.x * g0 + da.y * g1 + da.z * g2) * m;
+            } else {
+                const float4 wb = wbs[t];
+                tv1 += (g0 * (wa.x - wb.x) + g1 * (wa.y - wb.y) + g2 * (wa.z - wb.z)) * fm0 * dt;
+                tv2 += ((da.x - g0 * qd) * g0 + (da.y - g1 * qd) * g1 + (da.z - g2 * qd) * g2) * fm0;
+            }
+        });
     if (tv2 == 0.f) tv2 = 1.f;
     reinterpret_cast<float*>(s.cC + p)[3] = tv2;
     s.aux1[p] = ra + tv1;
@@ -677,43 +688,48 @@ __global__ void __launch_bounds__(NT) k_ii_force(DevScene s, SolverConst c, int 
         const float den0 = 0.01f * c.hs * c.hs;
         float px = 0.f, py = 0.f, pz = 0.f;
         const int cnt = s.ncount[p];
-        const size_t stride = (size_t)c.stride;
-        for (int k = 0; k < cnt; ++k) {
-            bool bnd;
-            unsigned j;
-            nbr_fetch(s, (unsigned)ell_get(s.nbr, stride, p, k), bnd, j);
-            const float4 pb = bnd ? s.bpos[j] : s.pos[j];
-            const float xx = pa.x - pb.x, xy = pa.y - pb.y, xz = pa.z - pb.z;
-            const float len2 = xx * xx + xy * xy + xz * xz;
-            if (len2 == 0.f) { ++zero; continue; }
-            const float f = grad_over_r(c.k, len2);
-            float acce;
-            if (bnd) {
-                if (!(pra > 0.f)) continue;
-                acce = f * (-rho0 * pb.w * (pra / (ra * ra) * 2.f));
-            } else {
-                const float rb = s.cB[j].w, prb = s.kr[j];
-                const int phb = phase_of(pb);
-                if (phb == ph) {
-                    acce = f * (-fm0 * (pra / (ra * ra) + prb / (rb * rb)));
+        // a fluid neighbour's record {position, (p_l, rho)} as the phases'
+        // loops left it (p_l is its pressure)
+        float4 pbs[4], rbs[4];
+        walk4(
+            s.nbr, (size_t)c.stride, p, cnt, (unsigned)p, l2_policy(c.l2pol & 3),
+            [&](int t, unsigned u) {
+                ld_record32((u & BND_FLAG ? s.bpv : s.prv) + 2 * (size_t)(u & BND_MASK), pbs[t], rbs[t]);
+            },
+            [&](int t, unsigned u) {
+                const bool bnd = (u & BND_FLAG) != 0u;
+                const float4 pb = pbs[t];
+                const float xx = pa.x - pb.x, xy = pa.y - pb.y, xz = pa.z - pb.z;
+                const float len2 = xx * xx + xy * xy + xz * xz;
+                if (len2 == 0.f) { ++zero; return; }
+                const float f = grad_over_r(c.k, len2);
+                float acce;
+                if (bnd) {
+                    if (!(pra > 0.f)) return;
+                    acce = f * (-rho0 * pb.w * (pra / (ra * ra) * 2.f));
                 } else {
-                    const float fmb = c.fm_ph[phb];
-                    const float da = ra / fm0, db = rb / fmb;
-                    acce = f * (-1.f / fm0 * (pra / (da * da) + prb / (db * db)));
-                    const float4 vb = s.vel[j];
-                    const float pro = (va.x - vb.x) * xx + (va.y - vb.y) * xy + (va.z - vb.z) * xz;
-                    if (pro < 0.f) {
-                        const float al = (alpha + c.alpha_ph[phb]) / 2.f;
-                        const float nu = 2.f * al * c.hs * c.cs / (ra + rb);
-                        const float pi = -nu * pro / (len2 + den0);
-                        acce += f * (-(fm0 + fmb) / 2.f * pi);
+                    const float rb = rbs[t].y, prb = rbs[t].x;
+                    const int phb = phase_of(pb);
+                    if (phb == ph) {
+                        acce = f * (-fm0 * (pra / (ra * ra) + prb / (rb * rb)));
+                    } else {
+                        const float fmb = c.fm_ph[phb];
+                        const float da = ra / fm0, db = rb / fmb;
+                        acce = f * (-1.f / fm0 * (pra / (da * da) + prb / (db * db)));
+                        const float4 vb = s.vel[u];
+                        const float pro = (va.x - vb.x) * xx + (va.y - vb.y) * xy + (va.z - vb.z) * xz;
+                        if (pro < 0.f) {
+                            const float al = (alpha + c.alpha_ph[phb]) / 2.f;
+                            const float nu = 2.f * al * c.hs * c.cs / (ra + rb);
+                            const float pi = -nu * pro / (len2 + den0);
+                            acce += f * (-(fm0 + fmb) / 2.f * pi);
+                        }
                     }
                 }
-            }
-            px = fmaf(xx, acce, px);
-            py = fmaf(xy, acce, py);
-            pz = fmaf(xz, acce, pz);
-        }
+                px = fmaf(xx, acce, px);
+                py = fmaf(xy, acce, py);
+                pz = fmaf(xz, acce, pz);
+            });
         s.acc[p] = make_float4(px, py, pz, 0.f);
         const float4 ca = s.cA[p];
         float4 v = (compat & 2) ? va : make_float4(ca.x, ca.y, ca.z, 0.f);
