@@ -452,17 +452,24 @@ __global__ void __launch_bounds__(NT, 8) k_ii_density(DevScene s, SolverConst c,
     if (threadIdx.x == 0 && cntb) atomicAdd(&s.st->ii_num, cntb);
 }
 
+// m_k p_j / rho_j^2 of IISph_M.cpp:300 for the phase being solved: a function
+// of the neighbour alone, divided once per particle instead of once per pair
+__device__ __forceinline__ float ii_p_term(float fm0, float pl, float rho) { return (fm0 * pl) / (rho * rho); }
+
 // a_ii, rho_adv, p_l = p/2 (IISph_M.cpp:243-278)
 __global__ void __launch_bounds__(NT, 8) k_ii_aii(DevScene s, SolverConst c, int phase) {
     const int n = s.st->n_active;
     const int p = blockIdx.x * NT + threadIdx.x;
     if (p >= n) return;
     const float4 pa = s.pos[p];
-    // every particle's record for the sum sweep of this phase's loop:
-    // {position, (p_l, rho)} (the other phases keep their carried values)
+    // every particle's record for the sum sweep of this phase's loop, (x, y,
+    // z, m_k p_l / rho^2) (the other phases keep their carried values), and
+    // for the pressure force, {position, (p_l, rho)}
     s.prv[2 * p] = pa;
     if (phase_of(pa) != phase) {
-        s.prv[2 * p + 1] = make_float4(s.cA[p].w, s.cB[p].w, 0.f, 0.f);
+        const float pl = s.cA[p].w, rho = s.cB[p].w;
+        s.prv[2 * p + 1] = make_float4(pl, rho, 0.f, 0.f);
+        s.pk[p] = make_float4(pa.x, pa.y, pa.z, ii_p_term(c.fm_ph[phase], pl, rho));
         return;
     }
     const float dt = *s.dt;
@@ -506,14 +513,18 @@ __global__ void __launch_bounds__(NT, 8) k_ii_aii(DevScene s, SolverConst c, int
     const float pl = (float)(0.5 * (double)s.kr[p]);
     reinterpret_cast<float*>(s.cA + p)[3] = pl;
     s.prv[2 * p + 1] = make_float4(pl, ra, 0.f, 0.f);
+    s.pk[p] = make_float4(pa.x, pa.y, pa.z, ii_p_term(fm0, pl, ra));
 }
 
 // sum_j d_ij p_j = -dt^2 sum_f m_k p_j / rho_j^2 gradW (IISph_M.cpp:290-313);
-// every particle also saves its p_l as the previous iterate
-// Records: prv = {position, (p_l, rho)} (written by k_ii_aii for every
-// particle, p_l updated by k_ii_press), read here per fluid neighbour in one
-// 32-byte load; this kernel writes every particle's record for k_ii_press,
-// pv = {(d_ii, previous iterate p_l), (sum_j d_ij p_j, 0)}.
+// every particle also saves its p_l as the previous iterate.
+// A fluid neighbour is one 16-byte record pk = (x, y, z, m_k p_l / rho^2)
+// (written by k_ii_aii for every particle, w updated by k_ii_press); this
+// kernel writes every particle's record for k_ii_press, pv = {position,
+// d_ii p_l + sum_j d_ij p_j}, what a neighbour adds to the Jacobi sum.
+// Event-timed with k_ii_press, 32-byte record and a division per pair there,
+// position and 32-byte record here, before / now: 405 k particles 38.7 /
+// 26.4 and 52.6 / 40.8 us, 95 k 19.2 / 13.5 and 20.8 / 18.6.
 __global__ void __launch_bounds__(NT) k_ii_sum(DevScene s, SolverConst c, int phase) {
     const int n = s.st->n_active;
     const int p = blockIdx.x * NT + threadIdx.x;
@@ -525,42 +536,26 @@ __global__ void __launch_bounds__(NT) k_ii_sum(DevScene s, SolverConst c, int ph
     float4 cc = s.cC[p];
     if (phase_of(pa) == phase) {
         const float dt = *s.dt;
-        const float fm0 = c.fm_ph[phase];
         float tx = 0.f, ty = 0.f, tz = 0.f;
-        const int cnt = s.ncount[p];
-        const int ng = (cnt + 3) >> 2;
-        const size_t stride = (size_t)c.stride;
-        const unsigned long long polL = l2_policy(c.l2pol & 3);  // lists stream through L2
-        int4 nxt = ng ? ell_group_pol(s.nbr, stride, p, 0, polL) : make_int4(0, 0, 0, 0);
-        for (int gi = 0; gi < ng; ++gi) {
-            const int4 cur = nxt;
-            if (gi + 1 < ng) nxt = ell_group_pol(s.nbr, stride, p, gi + 1, polL);
-            const unsigned e[4] = {(unsigned)cur.x, (unsigned)cur.y, (unsigned)cur.z, (unsigned)cur.w};
-            float4 pb[4], rb[4];
-            bool use[4];
-#pragma unroll
-            for (int t = 0; t < 4; ++t) {
-                // boundary neighbours add nothing here: they read the own record
-                use[t] = gi * 4 + t < cnt && !(e[t] & BND_FLAG);
-                ld_record32(s.prv + 2 * (size_t)(use[t] ? e[t] : (unsigned)p), pb[t], rb[t]);
-            }
-#pragma unroll
-            for (int t = 0; t < 4; ++t) {
-                if (!use[t]) continue;
-                const float xx = pa.x - pb[t].x, xy = pa.y - pb[t].y, xz = pa.z - pb[t].z;
-                const float f = grad_over_r(c.k, xx * xx + xy * xy + xz * xz);
-                const float q = -(fm0 * rb[t].x) / (rb[t].y * rb[t].y) * f;
+        float4 pbs[4];
+        walk4(
+            s.nbr, (size_t)c.stride, p, s.ncount[p], (unsigned)p, l2_policy(c.l2pol & 3),
+            // boundary neighbours add nothing here: they read the own record
+            [&](int t, unsigned u) { pbs[t] = __ldg(s.pk + (u & BND_FLAG ? (unsigned)p : u)); },
+            [&](int t, unsigned u) {
+                if (u & BND_FLAG) return;
+                const float xx = pa.x - pbs[t].x, xy = pa.y - pbs[t].y, xz = pa.z - pbs[t].z;
+                const float q = -pbs[t].w * grad_over_r(c.k, xx * xx + xy * xy + xz * xz);
                 tx = fmaf(xx, q, tx);
                 ty = fmaf(xy, q, ty);
                 tz = fmaf(xz, q, tz);
-            }
-        }
+            });
         const float dt2 = dt * dt;
         cc = make_float4(tx * dt2, ty * dt2, tz * dt2, cc.w);
         s.cC[p] = cc;
     }
-    s.pv[2 * p] = make_float4(db.x, db.y, db.z, pla);
-    s.pv[2 * p + 1] = make_float4(cc.x, cc.y, cc.z, 0.f);
+    s.pv[2 * p] = pa;
+    s.pv[2 * p + 1] = make_float4(fmaf(db.x, pla, cc.x), fmaf(db.y, pla, cc.y), fmaf(db.z, pla, cc.z), 0.f);
 }
 
 // relaxed Jacobi update (IISph_M.cpp:315-351) and the loop decision (:352-358)
@@ -579,46 +574,31 @@ __global__ void __launch_bounds__(NT) k_ii_press(DevScene s, SolverConst c, int 
             const float ra = s.cB[p].w;
             const float pla = s.pl2[p];
             const float qd = dt * dt * fm0 / (ra * ra);
+            const float qp = qd * pla;
             float ft = 0.f;
-            const int cnt = s.ncount[p];
-            const int ng = (cnt + 3) >> 2;
-            const size_t stride = (size_t)c.stride;
-            const unsigned long long polL = l2_policy(c.l2pol & 3);  // lists stream through L2
-            // per fluid neighbour: its position and its k_ii_sum record
-            // {(d_jj, previous p_l), (sum_k d_jk p_k, 0)}; boundary: position
-            // and volume
-            int4 nxt = ng ? ell_group_pol(s.nbr, stride, p, 0, polL) : make_int4(0, 0, 0, 0);
-            for (int gi = 0; gi < ng; ++gi) {
-                const int4 cur = nxt;
-                if (gi + 1 < ng) nxt = ell_group_pol(s.nbr, stride, p, gi + 1, polL);
-                const unsigned e[4] = {(unsigned)cur.x, (unsigned)cur.y, (unsigned)cur.z, (unsigned)cur.w};
-                float4 pb[4], db[4], sb[4];
-                bool bnd[4];
-#pragma unroll
-                for (int t = 0; t < 4; ++t) {
-                    const unsigned u = gi * 4 + t < cnt ? e[t] : (unsigned)p;
-                    unsigned j;
-                    nbr_fetch(s, u, bnd[t], j);
-                    pb[t] = __ldg(bnd[t] ? s.bpos + j : s.pos + j);
-                    ld_record32(s.pv + 2 * (size_t)(bnd[t] ? (unsigned)p : j), db[t], sb[t]);
-                }
-#pragma unroll
-                for (int t = 0; t < 4; ++t) {
-                    if (gi * 4 + t >= cnt) break;
-                    const float xx = pa.x - pb[t].x, xy = pa.y - pb[t].y, xz = pa.z - pb[t].z;
+            // a fluid neighbour's k_ii_sum record, a boundary one's {(x, y, z,
+            // volume), v}
+            float4 pbs[4], ebs[4];
+            walk4(
+                s.nbr, (size_t)c.stride, p, s.ncount[p], (unsigned)p, l2_policy(c.l2pol & 3),
+                [&](int q, unsigned u) {
+                    ld_record32((u & BND_FLAG ? s.bpv : s.pv) + 2 * (size_t)(u & BND_MASK), pbs[q], ebs[q]);
+                },
+                [&](int q, unsigned u) {
+                    const float4 pb = pbs[q], eb = ebs[q];
+                    const float xx = pa.x - pb.x, xy = pa.y - pb.y, xz = pa.z - pb.z;
                     const float f = grad_over_r(c.k, xx * xx + xy * xy + xz * xz);
                     const float g0 = xx * f, g1 = xy * f, g2 = xz * f;
-                    if (bnd[t]) {
-                        ft += (rho0 * pb[t].w) * (ca.x * g0 + ca.y * g1 + ca.z * g2);
+                    if (u & BND_FLAG) {
+                        ft += (rho0 * pb.w) * (ca.x * g0 + ca.y * g1 + ca.z * g2);
                     } else {
-                        const float plb = db[t].w;
-                        const float t0 = (ca.x - db[t].x * plb) - (sb[t].x - g0 * qd * pla);
-                        const float t1 = (ca.y - db[t].y * plb) - (sb[t].y - g1 * qd * pla);
-                        const float t2 = (ca.z - db[t].z * plb) - (sb[t].z - g2 * qd * pla);
+                        // sum_j d_ij p_j - d_jj p_j - (sum_k d_jk p_k - d_ji p_i)
+                        const float t0 = fmaf(g0, qp, ca.x - eb.x);
+                        const float t1 = fmaf(g1, qp, ca.y - eb.y);
+                        const float t2 = fmaf(g2, qp, ca.z - eb.z);
                         ft += fm0 * (t0 * g0 + t1 * g1 + t2 * g2);
                     }
-                }
-            }
+                });
             const float aii = ca.w, radv = s.aux1[p];
             float t = (float)((1.0 - omega) * (double)pla + (omega / (double)aii) * (double)(rho0 - radv - ft));
             if (t < 0.f) {
@@ -630,7 +610,8 @@ __global__ void __launch_bounds__(NT) k_ii_press(DevScene s, SolverConst c, int 
             }
             reinterpret_cast<float*>(s.cA + p)[3] = t;
             s.kr[p] = t;
-            s.prv[2 * p + 1] = make_float4(t, ra, 0.f, 0.f);  // the next sum sweep's p_l
+            s.prv[2 * p + 1] = make_float4(t, ra, 0.f, 0.f);
+            s.pk[p].w = ii_p_term(fm0, t, ra);  // the next sum sweep's
         }
     }
     __shared__ double sh[NT / 32];
