@@ -27,16 +27,7 @@
 namespace {
 constexpr int NT = 128;
 
-// per-step counters (the last step's values are reported)
-__global__ void k_step_begin(DevScene s) {
-    DevStats* st = s.st;
-    st->max_nbrs = 0;
-    st->nbr_total = 0ull;
-    st->it_density = 0;
-    st->it_div = 0;
-    st->err_density = 0;
-    st->err_div = 0;
-}
+__global__ void k_step_begin(DevScene s) { stats_step_begin(s.st); }
 
 // per-call counters: status bits are OR-ed and removals / dropped pairs
 // summed over all steps of one API call
@@ -48,12 +39,6 @@ __global__ void k_call_begin(DevScene s) {
     st->status = 0u;
     st->total_it_density = 0;
     st->total_it_div = 0;
-}
-
-__global__ void k_loop_reset(DevScene s, int which) {
-    if (which == 0) s.st->it_density = 0;
-    else s.st->it_div = 0;
-    s.st->cont = 1;
 }
 
 // non-pressure accelerations (gravity + viscosity) and v_adv.  The list is
@@ -149,7 +134,8 @@ __device__ __forceinline__ void force_finish(const DevScene& s, const SolverCons
     }
 }
 template <int BS>
-__global__ void __launch_bounds__(BS) k_df_forces(DevScene s, SolverConst c, int warm) {
+__global__ void __launch_bounds__(BS) k_df_forces(DevScene s, SolverConst c, int warm, int begin) {
+    if (begin && blockIdx.x == 0 && threadIdx.x == 0) stats_step_begin(s.st);
     const int n = s.st->n_active;
     const int p = blockIdx.x * BS + threadIdx.x;
     int zero = 0;
@@ -541,7 +527,8 @@ __global__ void __launch_bounds__(BS) k_df_b_lanes(DevScene s, SolverConst c, in
 // non-pressure accelerations and v_adv (k_df_forces); a pair without a force
 // leaves a zero factor
 template <int BS>
-__global__ void __launch_bounds__(BS) k_df_forces_lanes(DevScene s, SolverConst c, int warm) {
+__global__ void __launch_bounds__(BS) k_df_forces_lanes(DevScene s, SolverConst c, int warm, int begin) {
+    if (begin && blockIdx.x == 0 && threadIdx.x == 0) stats_step_begin(s.st);
     __shared__ float term[BS / LANES][LROWS * 4];
     const int n = s.st->n_active;
     const int t = threadIdx.x % LANES, q = threadIdx.x / LANES;
@@ -652,7 +639,6 @@ static inline int nblk(int n, int bs = NT) { return (n > 0 ? n + bs - 1 : bs) / 
 
 void launch_step_begin(const DevScene& s, cudaStream_t st) { k_step_begin<<<1, 1, 0, st>>>(s); }
 void launch_call_begin(const DevScene& s, cudaStream_t st) { k_call_begin<<<1, 1, 0, st>>>(s); }
-void launch_df_loop_reset(const DevScene& s, int which, cudaStream_t st) { k_loop_reset<<<1, 1, 0, st>>>(s, which); }
 
 // the kernels with four threads per particle: 64 or 128 threads (their rows of
 // factors fit the default shared memory)
@@ -660,11 +646,12 @@ void launch_df_loop_reset(const DevScene& s, int which, cudaStream_t st) { k_loo
     if (bs == 64) { constexpr int B = 64; CALL; }       \
     else { constexpr int B = 128; CALL; }
 
-void launch_df_forces(const DevScene& s, const SolverConst& c, int n_max, int warm, cudaStream_t st, int bs) {
+void launch_df_forces(const DevScene& s, const SolverConst& c, int n_max, int warm, cudaStream_t st, int bs,
+                      bool begin) {
     if (c.lanes_a > 1) {
-        DISPATCH_LANES(bs, (k_df_forces_lanes<B><<<nblk(n_max, B / LANES), B, 0, st>>>(s, c, warm)));
+        DISPATCH_LANES(bs, (k_df_forces_lanes<B><<<nblk(n_max, B / LANES), B, 0, st>>>(s, c, warm, begin)));
     } else {
-        DISPATCH_BS(bs, (k_df_forces<B><<<nblk(n_max, B), B, 0, st>>>(s, c, warm)));
+        DISPATCH_BS(bs, (k_df_forces<B><<<nblk(n_max, B), B, 0, st>>>(s, c, warm, begin)));
     }
 }
 void launch_df_dens_a(const DevScene& s, const SolverConst& c, int n_max, int record, cudaStream_t st, int bs) {

@@ -131,6 +131,7 @@ struct sphgpu_scene {
     // the list build (SolverConst::build): -1 by size, else 0 or 1 (debug knob "build")
     int build = -1;
     int sweep_lanes = 0;  // SolverConst::lanes_a, lanes_b: 0 by size, 1 or 4 (debug knob "sweep_lanes")
+    int scan_max = SCAN_MAX;  // cell keys scanned by one block (debug knob "scan": 0 CUB, else one block)
     int fuse_div = 1;  // DFSPH: the list build performs the divergence loop's first sweep A
     int fuse_ws = 1;   // warm start: features and inference in one kernel
     // set while a step that is not its call's last is enqueued: the step's
@@ -382,6 +383,7 @@ int alloc_scene(sphgpu_scene* h) {
     d.dt = &d.st->dt;
     d.nb = 0;
     cudaMemsetAsync(d.st, 0, sizeof(DevStats), h->stream);
+    cudaMemsetAsync(d.cell_count, 0, sizeof(int) * ((size_t)h->g.nkeys + 1), h->stream);
     cudaMemsetAsync(d.bcell_start, 0, sizeof(int) * ((size_t)h->g.nkeys + 1), h->stream);
     cudaMemsetAsync(d.ksum, 0, sizeof(float) * n, h->stream);
     cudaMemsetAsync(d.kwarm, 0, sizeof(float) * n, h->stream);
@@ -459,14 +461,17 @@ void enq_boundary_update(sphgpu_scene* h, cudaStream_t st) {
 
 void enq_ns(sphgpu_scene* h, int integrate, int build_mode, cudaStream_t st, int carry = 1) {
     DevScene& d = h->d;
-    cudaMemsetAsync(d.cell_count, 0, sizeof(int) * ((size_t)h->g.nkeys + 1), st);
+    // (the counts are zero: at first, and after every scatter)
     launch(h, "hash", st, [&] { launch_hash(d, h->g, integrate, h->cap, st); });
     launch(h, "scan", st, [&] {
+        if (h->g.nkeys + 1 <= h->scan_max) {
+            launch_scan(d, h->g, st);
+            return;
+        }
         size_t b = h->cub_bytes;
         cub::DeviceScan::ExclusiveSum(h->cub_tmp, b, d.cell_count, d.cell_start, h->g.nkeys + 1, st);
     });
     launch(h, "reorder", st, [&] { launch_scatter_reorder(d, h->g, h->cap, carry, st); });
-    launch_count_active(d, h->g, st);
     if (h->nscenes > 1) launch_batch_count(d, h->nscenes, st);
     if (h->R.nd)
         launch(h, "rigid_volume", st,
@@ -532,7 +537,6 @@ int enq_loop(sphgpu_scene* h, bool capturing, Body&& body, Pre&& pre = NoPre(), 
 int enq_df_density_loop(sphgpu_scene* h, bool capturing) {
     DevScene& d = h->d;
     const SphParams& P = h->P;
-    launch_df_loop_reset(d, 0, h->stream);
     if (h->nscenes > 1) launch_batch_loop_reset(d, h->nscenes, 0, h->stream);
     return enq_loop(h, capturing, [&](cudaStream_t st, unsigned long long hd, int use) {
         launch(h, "df_density_a", st,
@@ -553,7 +557,6 @@ int enq_df_density_loop(sphgpu_scene* h, bool capturing) {
 int enq_df_div_loop(sphgpu_scene* h, bool capturing, bool fused = false) {
     DevScene& d = h->d;
     const SphParams& P = h->P;
-    launch_df_loop_reset(d, 1, h->stream);
     if (h->nscenes > 1) launch_batch_loop_reset(d, h->nscenes, 1, h->stream);
     // the velocity update and, for a batch, the per-scene decisions
     auto div_b_of = [&](int parts, cudaStream_t st, unsigned long long hd, int use) {
@@ -611,7 +614,6 @@ void enq_rigid_forces(sphgpu_scene* h, cudaStream_t st) {
 int enq_df_part1(sphgpu_scene* h, bool capturing) {
     DevScene& d = h->d;
     cudaStream_t st = h->stream;
-    launch_step_begin(d, st);
     // the boundary forces read the loop's summed stiffness; without the
     // warm start (whose post-processing clears the sum) it restarts here
     const bool dyn = h->R.nd > 0;
@@ -623,7 +625,7 @@ int enq_df_part1(sphgpu_scene* h, bool capturing) {
     else if (h->P.cfl)
         launch(h, "cfl", st, [&] { launch_cfl(d, h->cap, h->P.cfl_factor, h->P.particle_d, h->P.dt_max, h->P.dt_min, st); });
     const int ws = h->mlp ? h->ws_mode : 0;
-    launch(h, "df_forces", st, [&] { launch_df_forces(d, h->c, h->cap, 0, st, h->tune.forces); });
+    launch(h, "df_forces", st, [&] { launch_df_forces(d, h->c, h->cap, 0, st, h->tune.forces, true); });
     if (h->P.enable_vortex)
         launch(h, "vortex", st, [&] {
             launch_vortex_second(d, h->c, h->P.enable_vortex, h->P.vort_alpha, h->P.vort_zeta, h->P.vort_nu_t,
@@ -734,11 +736,9 @@ int enq_pci_step(sphgpu_scene* h, bool capturing) {
     DevScene& d = h->d;
     cudaStream_t st = h->stream;
     const SphParams& P = h->P;
-    launch_step_begin(d, st);
-    enq_ns(h, 0, 0, st, 4);
+    enq_ns(h, 8, 0, st, 4);
     const float delta = pci_delta(P, h->c.k);
     launch(h, "pci_force_except", st, [&] { launch_pci_force_except(d, h->c, h->cap, st); });
-    launch_df_loop_reset(d, 0, st);
     int r = enq_loop(h, capturing, [&](cudaStream_t s2, unsigned long long hd, int use) {
         launch(h, "pci_density", s2, [&] { launch_pci_density(d, h->c, delta, h->cap, s2); });
         launch(h, "pci_pressure", s2, [&] {
@@ -757,8 +757,7 @@ int enq_ii_step(sphgpu_scene* h, bool capturing) {
     DevScene& d = h->d;
     cudaStream_t st = h->stream;
     const SphParams& P = h->P;
-    launch_step_begin(d, st);
-    enq_ns(h, 0, 0, st, 2 | 4 | 8);
+    enq_ns(h, 8, 0, st, 2 | 4 | 8);
     launch(h, "ii_force_except", st, [&] { launch_ii_force_except(d, h->c, h->cap, st); });
     const int nph = (int)h->rho0_ph.size();
     for (int ph = 0; ph < nph; ++ph) {
@@ -801,9 +800,9 @@ int ensure_iv_boundary(sphgpu_scene* h) {
 // neighbour lists of fluid and boundary particles with IISph's
 // DF_prepareAttribute / VF_prepareAttribute terms (IISph.cpp:100-545); the
 // carried loop velocity (cA) and stiffnesses (cC) follow the reorder
-void enq_iv_prepare(sphgpu_scene* h, bool from_staging, cudaStream_t st) {
+void enq_iv_prepare(sphgpu_scene* h, bool from_staging, cudaStream_t st, int begin = 0) {
     DevScene& d = h->d;
-    if (from_staging) enq_ns(h, 0, 3, st, 2 | 8);
+    if (from_staging) enq_ns(h, begin, 3, st, 2 | 8);
     else launch(h, "build_iisph", st, [&] { launch_build(d, h->g, h->c, 3, h->cap, st, h->tune.build); });
     launch(h, "iv_boundary_build", st, [&] { launch_iv_boundary_build(d, h->g, h->c, h->tune.build, st); });
 }
@@ -838,8 +837,7 @@ int enq_iv_loops(sphgpu_scene* h, bool capturing, int div) {
 int enq_iv_step(sphgpu_scene* h, bool capturing) {
     DevScene& d = h->d;
     cudaStream_t st = h->stream;
-    launch_step_begin(d, st);
-    enq_iv_prepare(h, true, st);
+    enq_iv_prepare(h, true, st, 8);
     launch(h, "iv_forces", st, [&] { launch_iv_forces(d, h->c, h->cap, h->tune.forces, st); });
     int r = enq_iv_loops(h, capturing, 1);
     if (r) return r;
@@ -856,8 +854,7 @@ int enq_iv_step(sphgpu_scene* h, bool capturing) {
 // copy sits on the step's critical path: 75 -> 69 us per step at 27 k)
 int enq_wc_step(sphgpu_scene* h, bool, bool copy_stats = true) {
     cudaStream_t st = h->stream;
-    launch_step_begin(h->d, st);
-    enq_ns(h, 0, 2, st);
+    enq_ns(h, 8, 2, st);
     const bool surf = h->P.th_h != 0.f || h->P.th_r != 0.f || h->P.th_bt != 0.f;
     if (surf) launch(h, "wc_normal", st, [&] { launch_wc_normal(h->d, h->c, h->cap, st); });
     launch(h, "wc_force", st, [&] { launch_wc_force(h->d, h->c, h->cap, st, surf, h->c.lanes); });
@@ -2233,8 +2230,8 @@ int sphgpu_stage(sphgpu_t h, const char* name, SphStepStats* stats) {
         enq_rigid_forces(h, st);
         if (dyn && h->mlp && h->ws_mode == 1) launch_ws_post(d, h->c, nullptr, h->cap, st);
         // integrate into staging (the reference updates positions in place)
-        cudaMemsetAsync(d.cell_count, 0, sizeof(int) * ((size_t)h->g.nkeys + 1), st);
         launch_hash(d, h->g, h->P.enable_vortex ? 3 : 1, h->cap, st);
+        cudaMemsetAsync(d.cell_count, 0, sizeof(int) * ((size_t)h->g.nkeys + 1), st);  // no sort follows
         h->ep_acc = h->ep_loop = h->sorts;
         if (h->P.enable_vortex == 1 || h->P.enable_vortex == 2) h->ep_vort = h->sorts;
         h->in_staging = true;
@@ -2927,6 +2924,7 @@ int sphgpu_get_solid_force(sphgpu_t h, int solid_id, double force[3], double tor
 //   fuse_div               DFSPH: the list build runs the divergence loop's first sweep A
 //   sweep_lanes            threads per particle of the DFSPH sweeps (0 by size, 1, 4)
 //   build                  list build (-1 by size, 0 a thread per particle, 1 a warp for a few)
+//   scan                   cell-count scan: 0 CUB over the chip, else one block
 //   fuse_ws                warm start: feature gather and network in one kernel
 //   speculative_host_step  sphgpu_step_host runs part 1 while checking its inputs
 //   wc_lanes               WCSPH threads per particle (0 by size, 1, 4)
@@ -2949,6 +2947,7 @@ int sphgpu_debug_set(sphgpu_t h, const char* key, int value) {
         invalidate_graphs(h);
         return 0;
     }
+    if (k == "scan") { h->scan_max = value ? 0x7fffffff : 0; invalidate_graphs(h); return 0; }
     if (k == "fuse_ws") { h->fuse_ws = value != 0; invalidate_graphs(h); return 0; }
     if (k == "wc_lanes") {
         if (value != 0 && value != 1 && value != 4) return SPHGPU_EINVAL;

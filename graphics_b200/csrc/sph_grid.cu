@@ -26,12 +26,15 @@ constexpr int NT = 256;
 
 __global__ void __launch_bounds__(NT) k_hash(DevScene s, GridGeom g, int integrate) {
     const int n = s.st->n_active;
-    if (blockIdx.x == 0 && threadIdx.x == 0) s.st->pad0 = n;  // staged count
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        s.st->pad0 = n;  // staged count
+        if (integrate & 8) stats_step_begin(s.st);
+    }
     int i = blockIdx.x * NT + threadIdx.x;
     int removed = 0, nan = 0;
     if (i < n) {
         float4 p, v;
-        if (integrate) {
+        if (integrate & 7) {
             // Second loop 2.4: velocity = vel_adv; position += velocity*dt
             // (DFSPH.cpp:705-715), in round-to-nearest float ops.
             p = s.pos[i];
@@ -82,10 +85,75 @@ __global__ void __launch_bounds__(NT) k_hash(DevScene s, GridGeom g, int integra
     }
 }
 
-__global__ void __launch_bounds__(NT) k_scatter(DevScene s) {
+// Everything that needs the cell starts only: the particles' arrival slots,
+// the interleaved {fluid start, boundary start} per cell key (one 8-byte load
+// per cell bound in the list build), the number of active particles, and the
+// counts back to zero for the next search.
+__global__ void __launch_bounds__(NT) k_scatter(DevScene s, int nk) {
     const int n = s.st->pad0;
-    int i = blockIdx.x * NT + threadIdx.x;
+    const int i = blockIdx.x * NT + threadIdx.x;
     if (i < n) s.tmp[s.cell_start[s.key[i]] + s.slot[i]] = i;
+    if (i <= nk) {
+        s.cstart2[i] = make_int2(s.cell_start[i], s.bcell_start[i]);
+        s.cell_count[i] = 0;
+    }
+    if (i == 0) {
+        const int act = s.cell_start[nk - 1];  // the dead key's start
+        s.st->removed += n - act;
+        s.st->n_active = act;
+    }
+}
+
+// Exclusive scan of n counts by one block: 4096 a round, the next round's
+// loads issued before the current one is summed.
+constexpr int SCAN_NT = 1024;
+__global__ void __launch_bounds__(SCAN_NT) k_scan(const int* __restrict__ in, int* __restrict__ out, int n) {
+    __shared__ int wsum[SCAN_NT / 32];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    auto load = [&](int i) {
+        int4 v = make_int4(0, 0, 0, 0);
+        if (i + 3 < n) {
+            v = *reinterpret_cast<const int4*>(in + i);
+        } else {
+            if (i < n) v.x = in[i];
+            if (i + 1 < n) v.y = in[i + 1];
+            if (i + 2 < n) v.z = in[i + 2];
+        }
+        return v;
+    };
+    int carry = 0;
+    int4 nxt = load(4 * threadIdx.x);
+    for (int base = 0; base < n; base += 4 * SCAN_NT) {
+        const int i = base + 4 * threadIdx.x;
+        const int4 v = nxt;
+        nxt = load(i + 4 * SCAN_NT);
+        const int sum = v.x + v.y + v.z + v.w;
+        int incl = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += t;
+        }
+        if (lane == 31) wsum[wid] = incl;
+        __syncthreads();
+        int w = wsum[lane];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, w, o);
+            if (lane >= o) w += t;
+        }
+        const int before = carry + (wid ? __shfl_sync(0xffffffffu, w, wid - 1) : 0) + incl - sum;
+        carry += __shfl_sync(0xffffffffu, w, 31);
+        __syncthreads();
+        const int4 o4 = make_int4(before, before + v.x, before + v.x + v.y, before + v.x + v.y + v.z);
+        if (i + 3 < n) {
+            *reinterpret_cast<int4*>(out + i) = o4;
+        } else {
+            if (i < n) out[i] = o4.x;
+            if (i + 1 < n) out[i + 1] = o4.y;
+            if (i + 2 < n) out[i + 2] = o4.z;
+        }
+    }
 }
 
 // For sorted slot q: its particle i, its cell range [a, b); its final place is
@@ -121,15 +189,8 @@ __global__ void __launch_bounds__(NT) k_rank_reorder(DevScene s, int dead_key, i
     if (carry & 8) s.cC[p] = s.cC_s[i];
 }
 
-// interleaved {fluid start, boundary start} per cell key: one 8-byte load
-// per cell bound in the neighbour-list kernel
-// dead_key >= 0: also the number of active particles
-__global__ void k_merge_starts(DevScene s, int nk, int dead_key) {
-    if (dead_key >= 0 && blockIdx.x == 0 && threadIdx.x == 0) {
-        const int staged = s.st->pad0, act = s.cell_start[dead_key];
-        s.st->removed += staged - act;
-        s.st->n_active = act;
-    }
+// the interleaved starts again after the boundary alone was re-sorted
+__global__ void k_merge_starts(DevScene s, int nk) {
     const int k = blockIdx.x * NT + threadIdx.x;
     if (k <= nk) s.cstart2[k] = make_int2(s.cell_start[k], s.bcell_start[k]);
 }
@@ -500,18 +561,18 @@ void launch_hash(const DevScene& s, const GridGeom& g, int integrate, int n_old,
     k_hash<<<nblk(n_old > 0 ? n_old : 1, NT), NT, 0, st>>>(s, g, integrate);
 }
 
-void launch_scatter_reorder(const DevScene& s, const GridGeom& g, int n_old, int carry, cudaStream_t st) {
-    int nb = nblk(n_old > 0 ? n_old : 1, NT);
-    k_scatter<<<nb, NT, 0, st>>>(s);
-    k_rank_reorder<<<nb, NT, 0, st>>>(s, g.nkeys - 1, carry);
+void launch_scan(const DevScene& s, const GridGeom& g, cudaStream_t st) {
+    k_scan<<<1, SCAN_NT, 0, st>>>(s.cell_count, s.cell_start, g.nkeys + 1);
 }
 
-void launch_count_active(const DevScene& s, const GridGeom& g, cudaStream_t st) {
-    k_merge_starts<<<nblk(g.nkeys + 1, NT), NT, 0, st>>>(s, g.nkeys, g.nkeys - 1);
+void launch_scatter_reorder(const DevScene& s, const GridGeom& g, int n_old, int carry, cudaStream_t st) {
+    const int n = n_old > 0 ? n_old : 1;
+    k_scatter<<<nblk(n > g.nkeys + 1 ? n : g.nkeys + 1, NT), NT, 0, st>>>(s, g.nkeys);
+    k_rank_reorder<<<nblk(n, NT), NT, 0, st>>>(s, g.nkeys - 1, carry);
 }
 
 void launch_merge_starts(const DevScene& s, const GridGeom& g, cudaStream_t st) {
-    k_merge_starts<<<nblk(g.nkeys + 1, NT), NT, 0, st>>>(s, g.nkeys, -1);
+    k_merge_starts<<<nblk(g.nkeys + 1, NT), NT, 0, st>>>(s, g.nkeys);
 }
 
 template <int BS, bool STAGED>

@@ -170,6 +170,16 @@ struct RigidDev {
     int nb, nd;
 };
 
+// per-step counters (the last step's values are reported), by one thread
+__device__ __forceinline__ void stats_step_begin(DevStats* st) {
+    st->max_nbrs = 0;
+    st->nbr_total = 0ull;
+    st->it_density = 0;
+    st->it_div = 0;
+    st->err_density = 0;
+    st->err_div = 0;
+}
+
 // step length of the particle's scene
 __device__ __forceinline__ float dt_of(const DevScene& s, float4 pa) {
     return s.nscenes > 1 ? s.b.dt[scene_of(pa)] : *s.dt;
@@ -267,12 +277,17 @@ __device__ __forceinline__ void walk4(const int* list, size_t stride, int p, int
 
 // ---- neighbour search (sph_grid.cu) ----
 // integrate: bit 0 the DFSPH position update, bit 1 carry cA, bit 2 the
-// learned warm start's history from this step's sums (k_ws_post's job)
+// learned warm start's history from this step's sums (k_ws_post's job), bit 3
+// the step begins here (stats_step_begin)
 void launch_hash(const DevScene& s, const GridGeom& g, int integrate, int n_old, cudaStream_t st);
-// carry: bit 0 hist, bit 1 cA, bit 2 cB, bit 3 cC (staging -> sorted)
+// carry: bit 0 hist, bit 1 cA, bit 2 cB, bit 3 cC (staging -> sorted); also the
+// active count, the interleaved cell starts, and the counts back to zero
 void launch_scatter_reorder(const DevScene& s, const GridGeom& g, int n_old, int carry, cudaStream_t st);
-// active count and the interleaved cell starts
-void launch_count_active(const DevScene& s, const GridGeom& g, cudaStream_t st);
+// exclusive scan of the cell counts by one block, up to SCAN_MAX keys; above,
+// CUB's two launches over the chip (WCSPH step with CUB / one block: 24.7 /
+// 22.7 us at 1.7 k keys, 32.0 / 31.2 at 4 k, 47.4 / 47.3 at 8 k, 84 / 90 at 14 k)
+constexpr int SCAN_MAX = 1 << 13;
+void launch_scan(const DevScene& s, const GridGeom& g, cudaStream_t st);
 // ---- list build, a warp per particle (sph_warp.cu) ----
 void launch_warp_build(const DevScene& s, const GridGeom& g, const SolverConst& c, int mode, int n_max, cudaStream_t st,
                        int bs);
@@ -301,7 +316,9 @@ void launch_boundary_volume(const DevScene& s, const GridGeom& g, float dpart, f
 
 // ---- DFSPH (sph_dfsph.cu) ----
 // bs: threads per block (64, 128 or 256; the autotuner's choice)
-void launch_df_forces(const DevScene& s, const SolverConst& c, int n_max, int warm, cudaStream_t st, int bs = 128);
+// begin: the step begins here (stats_step_begin)
+void launch_df_forces(const DevScene& s, const SolverConst& c, int n_max, int warm, cudaStream_t st, int bs = 128,
+                      bool begin = false);
 void launch_df_dens_a(const DevScene& s, const SolverConst& c, int n_max, int record, cudaStream_t st, int bs = 128);
 // blocks of part A (or of the list build with the first divergence sweep):
 // the FP64 partials that part B's decision adds up (its `parts`)
@@ -314,7 +331,6 @@ void launch_df_div_b(const DevScene& s, const SolverConst& c, int n_max, int par
                      int min_it, int max_it, unsigned long long cond_handle, int use_handle, cudaStream_t st,
                      int bs = 128);
 void launch_df_warm_correction(const DevScene& s, const SolverConst& c, int n_max, cudaStream_t st, int bs = 128);
-void launch_df_loop_reset(const DevScene& s, int which, cudaStream_t st);
 void launch_cfl(const DevScene& s, int n_max, float cfl, float d, float dt_max, float dt_min, cudaStream_t st);
 void launch_step_begin(const DevScene& s, cudaStream_t st);
 void launch_call_begin(const DevScene& s, cudaStream_t st);

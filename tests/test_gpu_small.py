@@ -130,3 +130,10 @@ def test_wcsph_plain_forces_match_the_general_pass(lanes, counts):
         g.close()
     # some 50 terms, each a few ulp of the largest, in either pass: 50 * 4 * 2^-24
     assert np.abs(acc[0] - acc[1]).max() <= 50 * 4 * 2.0 ** -24 * np.abs(acc[0]).max()
+
+
+# fewer cell keys than a round of the scan, several rounds with a remainder
+@pytest.mark.parametrize("counts", [(3, 3, 3), (29, 31, 33)])
+def test_one_block_scan_of_the_cell_counts(counts):
+    sc = _scene("block", counts)
+    _same(_run(sc, "dfsph", "scan", 0), _run(sc, "dfsph", "scan", 1))
