@@ -19,7 +19,7 @@
 
 struct MlpDev {
     float* master;          // FP32 parameters (Adam updates these)
-    float* grad;            // FP32 gradient of the last mini-batch
+    float* grad;            // FP32 gradient asked for by sphgpu_mlp_gradient
     float* gpart;           // [blocks][MLP_NPARAM_PAD] per-block gradients and
                             // [blocks] squared errors (after them): summed in a
                             // fixed order, so training is run-to-run deterministic
@@ -44,6 +44,8 @@ struct WsRecord {
 
 void launch_mlp_train_batch(const MlpDev& m, const float* X, const float* y, int n, int b0, int bsz, float inv_total,
                             cudaStream_t st);
-void launch_mlp_adam(const MlpDev& m, float lr, int t, cudaStream_t st);
+// after launch_mlp_train_batch of bsz rows: their gradient to m.grad, or one Adam step with it
+void launch_mlp_gradient(const MlpDev& m, int bsz, cudaStream_t st);
+void launch_mlp_adam(const MlpDev& m, int bsz, float lr, int t, cudaStream_t st);
 void launch_mlp_predict(const MlpDev& m, const float* X, float* y, int n, cudaStream_t st);
 void launch_mlp_sync_bf16(const MlpDev& m, cudaStream_t st);
