@@ -2552,7 +2552,7 @@ int sphgpu_mlp_train(sphgpu_mlp_t m, int epochs, int batch, float lr, float* los
         cudaMemsetAsync(m->m.loss, 0, sizeof(float), m->stream);
         for (int b0 = 0; b0 < n; b0 += batch) {
             const int bsz = std::min(batch, n - b0);
-            launch_mlp_train_batch(m->m, m->dsX, m->dsy, n, b0, bsz, 1.f / (float)bsz, m->stream);
+            launch_mlp_train_batch(m->m, m->dsX, m->dsy, n, b0, bsz, 1.f / (float)bsz, b0 > 0, m->stream);
             launch_mlp_adam(m->m, bsz, lr, ++m->adam_t, m->stream);
         }
         float l = 0;
@@ -2606,7 +2606,7 @@ int sphgpu_mlp_gradient(sphgpu_mlp_t m, const float* X, const float* y, int n, f
     copy_sync(dy, y, sizeof(float) * n, cudaMemcpyHostToDevice);
     cudaMemsetAsync(m->m.grad, 0, sizeof(float) * MLP_NPARAM_PAD, m->stream);
     cudaMemsetAsync(m->m.loss, 0, sizeof(float), m->stream);
-    launch_mlp_train_batch(m->m, dX, dy, n, 0, n, 1.f / (float)n, m->stream);
+    launch_mlp_train_batch(m->m, dX, dy, n, 0, n, 1.f / (float)n, false, m->stream);
     launch_mlp_gradient(m->m, n, m->stream);
     cudaMemcpyAsync(grad, m->m.grad, sizeof(float) * MLP_NPARAM, cudaMemcpyDeviceToHost, m->stream);
     float l = 0;

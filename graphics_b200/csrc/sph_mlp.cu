@@ -211,6 +211,12 @@ __device__ __forceinline__ void frag_bt(uint32_t r[4], const __nv_bfloat16* M, i
 constexpr int TNT = 512;  // threads of a training tile: 16 warps, 16 x 32 outputs each
 constexpr int XS = MLP_IN + 8, HS = MLP_H + 8, GS = MLP_H + 4;
 
+// programmatic dependent launch: what follows this in the kernel waits for the
+// kernel before it in the stream (at once when it was launched without), and
+// the next kernel may begin its own prologue
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_next() { asm volatile("griddepcontrol.launch_dependents;"); }
+
 struct TrainSmem {
     __nv_bfloat16 X[TR * XS];
     __nv_bfloat16 W1[MLP_IN * HS];
@@ -259,6 +265,11 @@ __global__ void __launch_bounds__(TNT) k_mlp_train(MlpDev m, const float* X, con
             make_uint2(pack2(__float2bfloat16_rn(x.x), __float2bfloat16_rn(x.y)),
                        pack2(__float2bfloat16_rn(x.z), __float2bfloat16_rn(x.w)));
     }
+    float target = 0.f;
+    const bool valid = tid < TR && tile0 + tid < end;
+    if (valid) target = (y[tile0 + tid] - m.norm[2 * MLP_IN]) * m.norm[2 * MLP_IN + 1];
+    pdl_wait();  // the rows are the dataset's; the weights are the update's
+    pdl_next();
     static_assert(TNT * 8 == MLP_H * MLP_H && TNT * 4 == TR * MLP_IN && MLP_OFF_W2 % 8 == 0, "one access per thread");
     *reinterpret_cast<uint4*>(&S.W2[(tid >> 3) * HS + (tid & 7) * 8]) =
         *reinterpret_cast<const uint4*>(m.w_bf16 + MLP_OFF_W2 + tid * 8);
@@ -272,9 +283,6 @@ __global__ void __launch_bounds__(TNT) k_mlp_train(MlpDev m, const float* X, con
         S.b2[i] = m.master[MLP_OFF_B2 + i];
     }
     if (tid == 0) S.b3 = m.master[MLP_OFF_B3];
-    float target = 0.f;
-    const bool valid = tid < TR && tile0 + tid < end;
-    if (valid) target = (y[tile0 + tid] - m.norm[2 * MLP_IN]) * m.norm[2 * MLP_IN + 1];
     __syncthreads();
 
     const int m0 = (w >> 1) * 16, n0 = (w & 1) * 32, ra = m0 + g, rb = ra + 8;
@@ -476,6 +484,8 @@ constexpr int UNT = 64;
 template <bool ADAM>
 __global__ void __launch_bounds__(UNT) k_mlp_update(MlpDev m, int blocks, float lr, float bc1, float bc2) {
     const int i = blockIdx.x * UNT + threadIdx.x;
+    pdl_wait();
+    pdl_next();
     if (blockIdx.x == gridDim.x - 1 && threadIdx.x >= UNT - 32) {
         // the last block's second warp has no parameter (static_assert below)
         const float* pl = m.gpart + (size_t)blocks * MLP_NPARAM_PAD;
@@ -557,18 +567,37 @@ void mlp_init_attributes() {
 
 int mlp_train_blocks(int bsz) { return (bsz + TR - 1) / TR; }
 
+// pdl: the kernel may start while the one before it in the stream ends
+template <class... P, class... A>
+static void launch_pdl(void (*k)(P...), int blocks, int threads, size_t smem, cudaStream_t st, bool pdl, A... args) {
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3(blocks);
+    c.blockDim = dim3(threads);
+    c.dynamicSmemBytes = smem;
+    c.stream = st;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = &at;
+    c.numAttrs = pdl;
+    cudaLaunchKernelEx(&c, k, static_cast<P>(args)...);
+}
+
 void launch_mlp_train_batch(const MlpDev& m, const float* X, const float* y, int n, int b0, int bsz, float inv_total,
-                            cudaStream_t st) {
-    k_mlp_train<<<mlp_train_blocks(bsz), TNT, smem_train(), st>>>(m, X, y, n, b0, bsz, inv_total);
+                            bool after_update, cudaStream_t st) {
+    launch_pdl(k_mlp_train, mlp_train_blocks(bsz), TNT, smem_train(), st, after_update, m, X, y, n, b0, bsz,
+               inv_total);
 }
 
 void launch_mlp_gradient(const MlpDev& m, int bsz, cudaStream_t st) {
-    k_mlp_update<false><<<(MLP_NPARAM + UNT - 1) / UNT, UNT, 0, st>>>(m, mlp_train_blocks(bsz), 0.f, 1.f, 1.f);
+    launch_pdl(k_mlp_update<false>, (MLP_NPARAM + UNT - 1) / UNT, UNT, 0, st, true, m, mlp_train_blocks(bsz), 0.f,
+               1.f, 1.f);
 }
 
 void launch_mlp_adam(const MlpDev& m, int bsz, float lr, int t, cudaStream_t st) {
     const float bc1 = 1.f - powf(0.9f, (float)t), bc2 = 1.f - powf(0.999f, (float)t);
-    k_mlp_update<true><<<(MLP_NPARAM + UNT - 1) / UNT, UNT, 0, st>>>(m, mlp_train_blocks(bsz), lr, bc1, bc2);
+    launch_pdl(k_mlp_update<true>, (MLP_NPARAM + UNT - 1) / UNT, UNT, 0, st, true, m, mlp_train_blocks(bsz), lr, bc1,
+               bc2);
 }
 
 void launch_mlp_sync_bf16(const MlpDev& m, cudaStream_t st) { k_mlp_sync<<<(MLP_NPARAM + 255) / 256, 256, 0, st>>>(m); }

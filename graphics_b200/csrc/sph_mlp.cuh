@@ -42,8 +42,10 @@ struct WsRecord {
     int ds_cap;
 };
 
+// after_update: the kernel before it in the stream is launch_mlp_adam's, and it
+// may read its rows while that one ends
 void launch_mlp_train_batch(const MlpDev& m, const float* X, const float* y, int n, int b0, int bsz, float inv_total,
-                            cudaStream_t st);
+                            bool after_update, cudaStream_t st);
 // after launch_mlp_train_batch of bsz rows: their gradient to m.grad, or one Adam step with it
 void launch_mlp_gradient(const MlpDev& m, int bsz, cudaStream_t st);
 void launch_mlp_adam(const MlpDev& m, int bsz, float lr, int t, cudaStream_t st);
