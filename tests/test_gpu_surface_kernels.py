@@ -69,3 +69,25 @@ def test_field_is_the_direct_sum(aniso, kind):
     # and a sum of up to a hundred kernels of both signs of error
     assert np.max(np.abs(got - want)) <= 2e-5 * np.max(want)
     sf.close()
+
+
+@pytest.mark.parametrize("ref_rows", [False, True])
+@pytest.mark.parametrize("box,share", [((0.15, 0.11, 0.13), 0.5), ((0.07, 0.3, 0.05), 0.02)])
+def test_marching_cubes_of_noise_is_the_restatement(ref_rows, box, share):
+    """Every cube case, blocks of cubes full of triangles and nearly empty
+    ones, rows that end within a thread's cubes: equal bit for bit."""
+    import mc_table as mt
+    from graphics_b200.surface import surface_field
+    sf = surface_field()
+    sf.surface_setup([0.0] * 3, box, R_P, R_H, R_P / 2)
+    num = [int(v) for v in sf.grid_num]
+    rng = np.random.default_rng(3)
+    f = rng.uniform(0, 1, num[::-1]).astype(np.float32)
+    f[rng.uniform(0, 1, f.shape) > share] += 1
+    sf.set_field(f)
+    got = sf.mesh(0.9, ref_rows=ref_rows)
+    want = mt.marching_cubes(f.ravel(), tuple(num), np.asarray(sf.grid_min, np.float32), np.float32(sf.cell_size), 0.9,
+                             ref_rows=ref_rows)
+    assert len(want) > 100
+    np.testing.assert_array_equal(got, want)
+    sf.close()
