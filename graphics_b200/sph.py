@@ -175,7 +175,9 @@ class GpuScene:
     def get(self, field):
         n = self.n_fluid
         comps = 3 if field in VEC_FIELDS else (_lib.MLP_IN if field == "ws_features" else 1)
-        out = np.zeros(max(n, 1) * comps, dtype=np.float32)
+        # not zeroed: the call writes all that is returned, and pages touched
+        # first by the copy cost twice the copy (119 070 particles: 344 -> 116 us)
+        out = np.empty(max(n, 1) * comps, dtype=np.float32)
         m = self._check(self.lib.sphgpu_get_fluid(self.h, field.encode(), _fptr(out)), "get " + field)
         return out[:m * comps].reshape(m, comps) if comps > 1 else out[:m]
 
