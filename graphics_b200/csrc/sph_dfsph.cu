@@ -488,7 +488,7 @@ __global__ void __launch_bounds__(BS) k_df_b_lanes(DevScene s, SolverConst c, in
         b_decide<BS, DIV>(s, c, parts, goal_abs, goal_rel, min_it, max_it, h, use_handle);
         return;
     }
-    __shared__ float term[BS / LANES][LROWS * 4];
+    __shared__ __align__(16) float term[BS / LANES][LROWS * 4];
     const int n = s.st->n_active;
     const int t = threadIdx.x % LANES, q = threadIdx.x / LANES;
     const int p = bid * (BS / LANES) + q;
@@ -529,7 +529,7 @@ __global__ void __launch_bounds__(BS) k_df_b_lanes(DevScene s, SolverConst c, in
 template <int BS>
 __global__ void __launch_bounds__(BS) k_df_forces_lanes(DevScene s, SolverConst c, int warm, int begin) {
     if (begin && blockIdx.x == 0 && threadIdx.x == 0) stats_step_begin(s.st);
-    __shared__ float term[BS / LANES][LROWS * 4];
+    __shared__ __align__(16) float term[BS / LANES][LROWS * 4];
     const int n = s.st->n_active;
     const int t = threadIdx.x % LANES, q = threadIdx.x / LANES;
     const int p = blockIdx.x * (BS / LANES) + q;
