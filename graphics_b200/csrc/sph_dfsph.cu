@@ -22,7 +22,7 @@
 // Loop control: k_*_b decides whether another iteration runs.  Inside a CUDA
 // graph the loop is a conditional WHILE node and the decision is written with
 // cudaGraphSetConditional; in host-driven mode it is written to st->cont.
-#include "sph_kernels.cuh"
+#include "sph_batch.cuh"
 
 namespace {
 constexpr int NT = 128;
@@ -251,10 +251,15 @@ __device__ __forceinline__ bool loop_goes_on(const SolverConst& c, double err, d
 // The block's part of the loop's FP64 error sum.  Part B, whose decision
 // needs it, adds the blocks up (b_decide): a last block that waited for the
 // others would end every part A with a chain of a fence, an atomic and the
-// loads (about 3 us).  A batch reduces per scene (k_batch_decide).
+// loads (about 3 us).  A batch reduces per scene (batch_decide); the sweep
+// hands its part B the flags it went by.
 template <int BS>
 __device__ __forceinline__ void a_partial(const DevScene& s, double mine) {
-    if (s.nscenes > 1) return;
+    if (s.nscenes > 1) {
+        if (blockIdx.x == 0)
+            for (int i = threadIdx.x; i < s.nscenes; i += BS) s.b.active_b[i] = s.b.active[i];
+        return;
+    }
     __shared__ double sh[BS / 32];
     const double b = block_sum_double<BS>(mine, sh);
     if (threadIdx.x == 0) s.partial[blockIdx.x] = b;
@@ -340,7 +345,8 @@ __device__ __forceinline__ void v_finish(const DevScene& s, int p, float4 va, fl
         s.prv[2 * p + 1] = va;
     }
 }
-// Part B's first block, which takes no particles: the error sum of part A's
+// Part B's first block, which takes no particles (its first `parts` ones for a
+// batch, DECIDE 2, run batch_decide): the error sum of part A's
 // `parts` blocks and the convergence decision of the iteration.
 template <int BS, int DIV>
 __device__ __forceinline__ void b_decide(const DevScene& s, const SolverConst& c, int parts, double goal_abs,
@@ -370,13 +376,19 @@ __global__ void __launch_bounds__(BS, 1152 / BS) k_df_vupdate(DevScene s, Solver
                                                    int min_it, int max_it, cudaGraphConditionalHandle h,
                                                    int use_handle) {
     int bid = blockIdx.x;
-    if (DECIDE && parts && bid-- == 0) {
+    if (DECIDE == 2) {
+        if (bid < parts) {
+            batch_decide<BS, DIV>(s, c, bid, parts, goal_abs, goal_rel, min_it, max_it, h, use_handle);
+            return;
+        }
+        bid -= parts;
+    } else if (DECIDE && parts && bid-- == 0) {
         b_decide<BS, DIV>(s, c, parts, goal_abs, goal_rel, min_it, max_it, h, use_handle);
         return;
     }
     const int n = s.st->n_active;
     const int p = bid * BS + threadIdx.x;
-    if (p < n && scene_active(s, s.pv[2 * p])) {
+    if (p < n && scene_active_b(s, s.pv[2 * p])) {
         const float dt = dt_of(s, s.pv[2 * p]);
         const float4 pa = s.pk[p];
         float dx = 0.f, dy = 0.f, dz = 0.f;
@@ -484,7 +496,13 @@ __global__ void __launch_bounds__(BS) k_df_b_lanes(DevScene s, SolverConst c, in
                                                    int min_it, int max_it, cudaGraphConditionalHandle h,
                                                    int use_handle) {
     int bid = blockIdx.x;
-    if (DECIDE && parts && bid-- == 0) {
+    if (DECIDE == 2) {
+        if (bid < parts) {
+            batch_decide<BS, DIV>(s, c, bid, parts, goal_abs, goal_rel, min_it, max_it, h, use_handle);
+            return;
+        }
+        bid -= parts;
+    } else if (DECIDE && parts && bid-- == 0) {
         b_decide<BS, DIV>(s, c, parts, goal_abs, goal_rel, min_it, max_it, h, use_handle);
         return;
     }
@@ -495,7 +513,7 @@ __global__ void __launch_bounds__(BS) k_df_b_lanes(DevScene s, SolverConst c, in
     int cnt = 0;
     float dt = 0.f;
     float4 va;
-    const bool act = p < n && scene_active(s, s.pv[2 * p]);
+    const bool act = p < n && scene_active_b(s, s.pv[2 * p]);
     if (act) {
         dt = dt_of(s, s.pv[2 * p]);
         va = s.pv[2 * p + 1];
@@ -670,8 +688,7 @@ static void launch_df_b(const DevScene& s, const SolverConst& c, int n_max, int 
                         int min_it, int max_it, unsigned long long cond_handle, int use_handle, cudaStream_t st,
                         int bs) {
     const cudaGraphConditionalHandle h = (cudaGraphConditionalHandle)cond_handle;
-    if (s.nscenes > 1) parts = 0;  // a batch decides per scene
-    const int extra = DECIDE && parts ? 1 : 0;
+    const int extra = DECIDE == 2 ? parts : (DECIDE && parts ? 1 : 0);
     if (c.lanes_b > 1) {
         DISPATCH_LANES(bs, (k_df_b_lanes<B, DIV, DECIDE><<<nblk(n_max, B / LANES) + extra, B, 0, st>>>(
                                s, c, parts, goal_abs, goal_rel, min_it, max_it, h, use_handle)));
@@ -682,6 +699,11 @@ static void launch_df_b(const DevScene& s, const SolverConst& c, int n_max, int 
 }
 void launch_df_dens_b(const DevScene& s, const SolverConst& c, int n_max, int parts, double goal, int min_it, int max_it,
                       unsigned long long cond_handle, int use_handle, cudaStream_t st, int bs) {
+    if (s.nscenes > 1) {  // a batch decides per scene
+        launch_df_b<0, 2>(s, c, n_max, batch_chunks(n_max, s.nscenes), 0.0, goal, min_it, max_it, cond_handle,
+                          use_handle, st, bs);
+        return;
+    }
     launch_df_b<0, 1>(s, c, n_max, parts, 0.0, goal, min_it, max_it, cond_handle, use_handle, st, bs);
 }
 void launch_df_warm_correction(const DevScene& s, const SolverConst& c, int n_max, cudaStream_t st, int bs) {
@@ -696,6 +718,11 @@ void launch_df_div_a(const DevScene& s, const SolverConst& c, int n_max, cudaStr
 }
 void launch_df_div_b(const DevScene& s, const SolverConst& c, int n_max, int parts, double goal_abs, double goal_rel,
                      int min_it, int max_it, unsigned long long cond_handle, int use_handle, cudaStream_t st, int bs) {
+    if (s.nscenes > 1) {  // a batch decides per scene
+        launch_df_b<1, 2>(s, c, n_max, batch_chunks(n_max, s.nscenes), goal_abs, goal_rel, min_it, max_it, cond_handle,
+                          use_handle, st, bs);
+        return;
+    }
     launch_df_b<1, 1>(s, c, n_max, parts, goal_abs, goal_rel, min_it, max_it, cond_handle, use_handle, st, bs);
 }
 // every block-size instantiation of the per-neighbour sweep kernels
@@ -707,6 +734,8 @@ static void each_sweep_kernel_bs(F f) {
     f((const void*)k_df_vupdate<B, 0, 1>);
     f((const void*)k_df_vupdate<B, 0, 0>);
     f((const void*)k_df_vupdate<B, 1, 1>);
+    f((const void*)k_df_vupdate<B, 0, 2>);
+    f((const void*)k_df_vupdate<B, 1, 2>);
 }
 template <int B, class F>
 static void each_lane_kernel_bs(F f) {
@@ -716,6 +745,8 @@ static void each_lane_kernel_bs(F f) {
     f((const void*)k_df_b_lanes<B, 0, 1>);
     f((const void*)k_df_b_lanes<B, 0, 0>);
     f((const void*)k_df_b_lanes<B, 1, 1>);
+    f((const void*)k_df_b_lanes<B, 0, 2>);
+    f((const void*)k_df_b_lanes<B, 1, 2>);
 }
 template <class F>
 static void each_sweep_kernel(F f) {

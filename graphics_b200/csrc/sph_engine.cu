@@ -545,11 +545,6 @@ int enq_df_density_loop(sphgpu_scene* h, bool capturing) {
             launch_df_dens_b(d, h->c, h->cap, df_a_blocks(h->c, h->cap, h->tune.sweep_a), P.df_density_goal, P.df_density_min_iter, P.df_density_max_iter, hd,
                              use, st, h->tune.sweep_b);
         });
-        if (h->nscenes > 1)
-            launch(h, "batch_decide", st, [&] {
-                launch_batch_decide(d, h->c, 0, h->nscenes, h->cap, 0.0, P.df_density_goal, P.df_density_min_iter,
-                                    P.df_density_max_iter, hd, use, st);
-            });
     });
 }
 
@@ -558,17 +553,11 @@ int enq_df_div_loop(sphgpu_scene* h, bool capturing, bool fused = false) {
     DevScene& d = h->d;
     const SphParams& P = h->P;
     if (h->nscenes > 1) launch_batch_loop_reset(d, h->nscenes, 1, h->stream);
-    // the velocity update and, for a batch, the per-scene decisions
     auto div_b_of = [&](int parts, cudaStream_t st, unsigned long long hd, int use) {
         launch(h, "df_div_b", st, [&] {
             launch_df_div_b(d, h->c, h->cap, parts, P.df_div_goal_abs, P.df_div_goal_rel, P.df_div_min_iter,
                             P.df_div_max_iter, hd, use, st, h->tune.sweep_b);
         });
-        if (h->nscenes > 1)
-            launch(h, "batch_decide", st, [&] {
-                launch_batch_decide(d, h->c, 1, h->nscenes, h->cap, P.df_div_goal_abs, P.df_div_goal_rel, P.df_div_min_iter,
-                                    P.df_div_max_iter, hd, use, st);
-            });
     };
     auto body = [&](cudaStream_t st, unsigned long long hd, int use) {
         launch(h, "df_div_a", st, [&] { launch_df_div_a(d, h->c, h->cap, st, h->tune.sweep_a); });
@@ -1380,7 +1369,7 @@ static int create_impl(const SphParams* p, int device, int max_fluid, int nscene
     if (!r && nscenes > 1) {
         // per-scene state: grids, then one block for the BatchDev arrays
         const size_t S = (size_t)nscenes;
-        const size_t bytes = S * (sizeof(float) + 9 * sizeof(int) + 3 * sizeof(double)) + 256 + sizeof(int);
+        const size_t bytes = S * (sizeof(float) + 10 * sizeof(int) + 3 * sizeof(double)) + 256 + sizeof(int);
         if (cudaMalloc((void**)&h->d_geom, S * sizeof(GridGeom)) != cudaSuccess ||
             cudaMalloc(&h->d_batch, bytes) != cudaSuccess) {
             r = SPHGPU_ENOMEM;
@@ -1394,6 +1383,7 @@ static int create_impl(const SphParams* p, int device, int max_fluid, int nscene
             b.vmax = (double*)q; q += S * sizeof(double);
             b.dt = (float*)q; q += S * sizeof(float);
             b.active = (int*)q; q += S * sizeof(int);
+            b.active_b = (int*)q; q += S * sizeof(int);
             b.it_density = (int*)q; q += S * sizeof(int);
             b.it_div = (int*)q; q += S * sizeof(int);
             b.total_it_density = (int*)q; q += S * sizeof(int);

@@ -39,6 +39,8 @@ struct BatchDev {
     const GridGeom* geom;  // [nscenes] grid of each scene (its key range)
     float* dt;             // [nscenes] step length
     int* active;           // [nscenes] 1 while the scene's current loop runs
+    int* active_b;         // [nscenes] as sweep A saw it: what sweep B reads while its
+                           // leading blocks decide (batch_decide)
     int* it_density;       // [nscenes] iterations of the last density / divergence loop
     int* it_div;
     int* total_it_density; // [nscenes] summed over the steps of the current call
@@ -187,6 +189,9 @@ __device__ __forceinline__ float dt_of(const DevScene& s, float4 pa) {
 // in a batch: is the particle's scene still iterating its current loop?
 __device__ __forceinline__ bool scene_active(const DevScene& s, float4 pa) {
     return s.nscenes <= 1 || s.b.active[scene_of(pa)] != 0;
+}
+__device__ __forceinline__ bool scene_active_b(const DevScene& s, float4 pa) {
+    return s.nscenes <= 1 || s.b.active_b[scene_of(pa)] != 0;
 }
 
 // This thread's share of the sum of n per-block partials, every BS-th in
@@ -338,9 +343,6 @@ void launch_call_begin(const DevScene& s, cudaStream_t st);
 // ---- batch of scenes (sph_batch.cu) ----
 void launch_batch_loop_reset(const DevScene& s, int nscenes, int which, cudaStream_t st);
 // n_cap: particle capacity (bounds the number of chunks)
-void launch_batch_decide(const DevScene& s, const SolverConst& c, int which, int nscenes, int n_cap, double goal_abs,
-                         double goal_rel, int min_it, int max_it, unsigned long long cond_handle, int use_handle,
-                         cudaStream_t st);
 void launch_batch_cfl(const DevScene& s, int nscenes, int n_cap, float cfl, float d, float dt_max, float dt_min,
                       cudaStream_t st);
 void launch_batch_call_begin(const DevScene& s, int nscenes, cudaStream_t st);
