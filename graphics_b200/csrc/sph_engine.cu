@@ -813,7 +813,7 @@ int enq_iv_loops(sphgpu_scene* h, bool capturing, int div) {
             launch(h, div ? "iv_div_a" : "iv_cv_a", s2,
                    [&] { launch_iv_sweep_a(d, h->c, ph, div, h->cap, h->tune.sweep_a, s2); });
             launch(h, div ? "iv_div_b" : "iv_cv_b", s2, [&] {
-                launch_iv_sweep_b(d, h->c, ph, div, goal, mn, mx, hd, use, h->cap, h->tune.sweep_b, s2);
+                launch_iv_sweep_b(d, h->c, ph, div, h->tune.sweep_a, goal, mn, mx, hd, use, h->cap, h->tune.sweep_b, s2);
             });
         });
         if (r) return r;

@@ -299,7 +299,7 @@ __global__ void __launch_bounds__(BS, STAGED ? 1024 / BS : 1) k_build(DevScene s
     }
     if (MODE == 4) {
         // the block's part of the iteration's FP64 sum of Drho/Dt (as
-        // k_df_div_a; a batch, mode 5, reduces per scene in k_batch_decide)
+        // k_df_div_a; a batch, mode 5, reduces per scene in batch_decide)
         __shared__ double shd[BS / 32];
         const double bsum = block_sum_double<BS>(ddiv, shd);
         if (threadIdx.x == 0) s.partial[blockIdx.x] = bsum;

@@ -212,30 +212,6 @@ __device__ __forceinline__ double partials_share(const double* partial, int n) {
     return acc;
 }
 
-// last-block FP64 reduction of per-block partials; returns true in the
-// thread that holds the total (thread 0 of the last block).  The partials
-// are summed in block order, so the total is the same from run to run.
-template <int BS>
-__device__ __forceinline__ bool finish_sum(double* partial, unsigned* ticket, double v, double* total) {
-    __shared__ bool last;
-    if (threadIdx.x == 0) {
-        partial[blockIdx.x] = v;
-        __threadfence();
-        unsigned t = atomicAdd(ticket, 1u);
-        last = (t == gridDim.x - 1);
-    }
-    __syncthreads();
-    if (!last) return false;
-    __threadfence();
-    __shared__ double sh[BS / 32];
-    double tot = block_sum_double<BS>(partials_share<BS>(partial, (int)gridDim.x), sh);
-    if (threadIdx.x == 0) {
-        *total = tot;
-        *ticket = 0u;
-    }
-    return threadIdx.x == 0;
-}
-
 // One pair's term of the DFSPH divergence sums, m_j gradW_ij . (v_i - v_j)
 // (DFSPH.cpp:589-617, 795-825) as the two factors t and m of its fma into
 // the sum: neighbour j's record {pb = (x, y, z, volume or phase), vb = loop
@@ -380,7 +356,7 @@ void launch_iv_phase_begin(const DevScene& s, cudaStream_t st);
 void launch_iv_loop_init(const DevScene& s, int phase, int div, int n_max, cudaStream_t st);
 void launch_iv_boundary_sweep(const DevScene& s, const SolverConst& c, int div, int bs, cudaStream_t st);
 void launch_iv_sweep_a(const DevScene& s, const SolverConst& c, int phase, int div, int n_max, int bs, cudaStream_t st);
-void launch_iv_sweep_b(const DevScene& s, const SolverConst& c, int phase, int div, double goal, int min_it,
+void launch_iv_sweep_b(const DevScene& s, const SolverConst& c, int phase, int div, int bs_a, double goal, int min_it,
                        int max_it, unsigned long long cond_handle, int use_handle, int n_max, int bs, cudaStream_t st);
 // acce_presure, v += acce_presure dt, x += v dt into the staging arrays (carried: v_adv)
 void launch_iv_integrate(const DevScene& s, int n_max, cudaStream_t st);

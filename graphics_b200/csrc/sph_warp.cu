@@ -232,7 +232,7 @@ __global__ void __launch_bounds__(BS) k_warp_build(const __grid_constant__ DevSc
     }
     if (MODE == 4) {
         // the block's part of the iteration's FP64 sum of Drho/Dt (as
-        // k_df_div_a; a batch, mode 5, reduces per scene in k_batch_decide)
+        // k_df_div_a; a batch, mode 5, reduces per scene in batch_decide)
         __shared__ double shd[WPB];
         const double bsum = block_sum_double<BS>(dsum, shd);
         if (threadIdx.x == 0) s.partial[blockIdx.x] = bsum;
