@@ -65,10 +65,10 @@ struct SolverConst {
     float ws_scale;    // applied fraction of the predicted warm-start stiffness
     int cap;           // neighbour cap
     int stride;        // ELL column stride (>= fluid capacity)
-    int build;         // list build: 0 a thread per particle (sph_grid.cu), 1 a warp for a few (sph_warp.cu)
+    int build;         // list build: 0 a thread per particle, 1 a warp for a few, 2 that for lists alone
     int lanes_a;       // threads per particle (1 or 4) of the DFSPH forces and A sweeps
     int lanes_b;       // and of the B sweeps
-    int lanes;         // threads per particle of the WCSPH list build and force pass (1 or 4)
+    int lanes;         // threads per particle of the WCSPH force pass (1 or 4)
     int l2pol;         // L2 eviction priority of the sweeps' loads: bits 0-1 the
                        // neighbour lists, bits 2-3 the gathered records
                        // (0 normal, 1 evict first, 2 evict last)

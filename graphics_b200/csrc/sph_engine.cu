@@ -137,8 +137,8 @@ struct sphgpu_scene {
     // set while a step that is not its call's last is enqueued: the step's
     // statistics stay on the device (the call's last step copies them)
     bool skip_stats = false;
-    // WCSPH threads per particle: 0 = by size (4 up to 262,144 particles of
-    // capacity, 1 above), else 1 or 4 (debug knob "wc_lanes")
+    // threads per particle of WCSPH's force pass: 0 by size (WC_LANES_MAX),
+    // else 1 or 4 (debug knob "wc_lanes")
     int wc_lanes = 0;
     // learned warm start: 0 off, 1 apply the network, 2 record training data
     sphgpu_mlp* mlp = nullptr;
@@ -258,9 +258,15 @@ GridGeom make_grid(const SphParams& P) {
 // particles (sph_warp.cu), larger ones with a thread per particle; measured,
 // thread / warp, event-timed: DFSPH rho + alpha + first divergence sweep 1 k
 // particles 52 / 14 us, 8 k 54 / 25, 27 k 57 / 41, 64 k 66 / 66, 125 k
-// - / 114 (thread 85); lists only 1 k 44 / 10, 64 k 54 / 37; WCSPH (4 threads
-// per particle) 27 k 34 / 31, 64 k 55 / 51
-constexpr int WARP_BUILD_MAX = 65536;
+// 85 / 114; WCSPH 27 k 48 / 28, 47 k 52 / 37, 64 k 55 / 57, 80 k 55 / 62,
+// 262 k 110 / 150.  Lists alone (PCISPH, IISPH_M) carry no sums that idle
+// lanes wait for: 1 k 44 / 10, 64 k 54 / 37, 97 k 57 / 45, 125 k 59 / 61, 166 k
+// 78 / 65, 262 k 99 / 98, 405 k 139 / 149
+constexpr int WARP_BUILD_MAX = 65536, WARP_LISTS_MAX = 262144;
+// WCSPH's force pass runs four threads per particle up to this capacity
+// (event-timed, one / four: 27 k 14.7 / 10.9 us, 47 k 15.9 / 14.6, 64 k 16.7 /
+// 16.7, 80 k 18.8 / 20.8, 262 k 40 / 46)
+constexpr int WC_LANES_MAX = 65536;
 // Capacities up to which the DFSPH sweeps run four threads per particle
 // (forces and the A sweeps; the B sweeps); both sides measured in sph_dfsph.cu
 constexpr int LANES_A_MAX = 24000, LANES_B_MAX = 12000;
@@ -300,10 +306,12 @@ void fill_solver_const(sphgpu_scene* h) {
     c.th_r = P.th_r;
     c.th_bt = P.th_bt;
     c.cap = h->ncap;
-    c.build = h->ncap <= 48 && (h->build < 0 ? h->cap <= WARP_BUILD_MAX : h->build != 0);
+    c.build = h->ncap > 48 ? 0
+              : h->build >= 0 ? h->build != 0
+                              : (h->cap <= WARP_BUILD_MAX ? 1 : (h->cap <= WARP_LISTS_MAX ? 2 : 0));
     c.stride = h->stride;
     c.l2pol = h->l2pol;
-    c.lanes = h->wc_lanes ? h->wc_lanes : (h->cap <= (1 << 18) ? 4 : 1);
+    c.lanes = h->wc_lanes ? h->wc_lanes : (h->cap <= WC_LANES_MAX ? 4 : 1);
     const bool lanes_ok = h->ncap <= 48;  // a particle's factors fit its shared-memory row
     c.lanes_a = lanes_ok && (h->sweep_lanes ? h->sweep_lanes == 4 : h->cap <= LANES_A_MAX) ? 4 : 1;
     c.lanes_b = lanes_ok && (h->sweep_lanes ? h->sweep_lanes == 4 : h->cap <= LANES_B_MAX) ? 4 : 1;
@@ -2918,7 +2926,7 @@ int sphgpu_get_solid_force(sphgpu_t h, int solid_id, double force[3], double tor
 //   scan                   cell-count scan: 0 CUB over the chip, else one block
 //   fuse_ws                warm start: feature gather and network in one kernel
 //   speculative_host_step  sphgpu_step_host runs part 1 while checking its inputs
-//   wc_lanes               WCSPH threads per particle (0 by size, 1, 4)
+//   wc_lanes               threads per particle of WCSPH's force pass (0 by size, 1, 4)
 int sphgpu_debug_set(sphgpu_t h, const char* key, int value) {
     if (!h || !key) return SPHGPU_EINVAL;
     std::string k(key);

@@ -306,112 +306,6 @@ __global__ void __launch_bounds__(BS, STAGED ? 1024 / BS : 1) k_build(DevScene s
     }
 }
 
-// WCSPH list build + density + Tait pressure (mode 2) with L threads per
-// particle, for small scenes (one thread per particle leaves too few warps
-// per SM to hide the candidate loads' latency).  Lane l scans a contiguous
-// range of the 27 cells in the reference's order into its own staged row;
-// the lanes' counts give each lane's offset in the particle's list, so the
-// list (and its cap) is the one-thread kernel's exactly.  Density: each
-// lane sums its kept entries, the partial sums are added in a fixed shuffle
-// order (deterministic; the one-thread kernel's sum is in list order).
-template <int L>
-__global__ void __launch_bounds__(128) k_build_wc_lanes(DevScene s, GridGeom g, SolverConst c) {
-    constexpr int BS = 128;
-    extern __shared__ int4 list_smem[];
-    int* const row = reinterpret_cast<int*>(list_smem) + threadIdx.x * LROW;
-    const int n = s.st->n_active;
-    const int t = blockIdx.x * BS + threadIdx.x;
-    const int p = t / L, l = t % L;
-    const bool act = p < n;
-    // lane l scans cells [c0, c1) of the 27
-    constexpr int PER = (27 + L - 1) / L;
-    const int c0 = l * PER, c1 = min(27, c0 + PER);
-    int cnt = 0;
-    float4 pa = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (act) {
-        pa = s.pos[p];
-        const GridGeom G = s.nscenes > 1 ? s.b.geom[scene_of(pa)] : g;
-        const int cx = cell_coord(pa.x, G.min[0], G.divisor);
-        const int cy = cell_coord(pa.y, G.min[1], G.divisor);
-        const int cz = cell_coord(pa.z, G.min[2], G.divisor);
-        const int cap = c.cap;
-        for (int ci = c0; ci < c1; ++ci) {
-            const int x = cx + ci % 3 - 1, y = cy + (ci / 3) % 3 - 1, z = cz + ci / 9 - 1;
-            if (!cell_inside(G, x, y, z)) continue;
-            const int key = cell_key(G, x, y, z);
-            const int2 s0 = __ldg(s.cstart2 + key), s1 = __ldg(s.cstart2 + key + 1);
-            for (int q = s0.x; q < s1.x; ++q) {
-                const float4 pb = __ldg(s.pos + q);
-                const float len2 = dis_square_rn(pa.x, pa.y, pa.z, pb.x, pb.y, pb.z);
-                const bool hit = len2 < c.h2cut && q != p;
-                if (hit && cnt < cap) row[cnt] = q;
-                cnt += hit;
-            }
-            for (int q = s0.y; q < s1.y; ++q) {
-                const float4 pb = __ldg(s.bpos + q);
-                const float len2 = dis_square_rn(pa.x, pa.y, pa.z, pb.x, pb.y, pb.z);
-                const bool hit = len2 < c.h2cut;
-                if (hit && cnt < cap) row[cnt] = q | (int)BND_FLAG;
-                cnt += hit;
-            }
-        }
-    }
-    // exclusive prefix of the lanes' counts within the particle's group
-    int pre = cnt;
-#pragma unroll
-    for (int off = 1; off < L; off <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, pre, off, L);
-        if (l >= off) pre += v;
-    }
-    const int total = __shfl_sync(0xffffffffu, pre, L - 1, L);
-    pre -= cnt;
-    const int cap = c.cap;
-    const int kept = min(total, cap);
-    float density = 0.f;
-    if (act) {
-        const size_t stride = (size_t)c.stride;
-        const int ph = phase_of(pa);
-        const float fm0 = c.fm_ph[ph], rho0 = c.rho0_ph[ph];
-        const int mine = max(0, min(cnt, cap - pre));
-        for (int i = 0; i < mine; ++i) {
-            const unsigned e = (unsigned)row[i];
-            s.nbr[ell_index(stride, p, pre + i)] = (int)e;
-            const bool bnd = (e & BND_FLAG) != 0u;
-            const float4 pb = __ldg((bnd ? s.bpos : s.pos) + (e & BND_MASK));
-            const float len2 = dis_square_rn(pa.x, pa.y, pa.z, pb.x, pb.y, pb.z);
-            float w, f;
-            kernel_pair(c.k, len2, w, f);
-            density = fmaf(bnd ? rho0 * pb.w : fm0, w, density);
-        }
-        if (l == 0) density = fmaf(ker_W(c.k, 0.f), fm0, density);
-    }
-#pragma unroll
-    for (int off = 1; off < L; off <<= 1) density += __shfl_xor_sync(0xffffffffu, density, off);
-    if (act && l == 0) {
-        const float rho0 = c.rho0_ph[phase_of(pa)];
-        s.ncount[p] = kept;
-        s.rho[p] = density;
-        // Tait, WcSph.cpp:142-146 (NEGLECT_NEGATIVE_PRESSURE)
-        float pr = c.wc_B * (powf(density / rho0, c.wc_gamma) - 1.f);
-        if (pr < 0.f) pr = 0.f;
-        s.kr[p] = pr;
-        // the force pass's record
-        const float4 v = s.vel[p];
-        s.prv[2 * p] = make_float4(pa.x, pa.y, pa.z, density);
-        s.prv[2 * p + 1] = make_float4(v.x, v.y, v.z, pr / (density * density));
-    }
-    __shared__ int sh[BS / 32];
-    const bool lead = act && l == 0;
-    int tot = block_sum_int<BS>(lead ? kept : 0, sh);
-    int ov = block_sum_int<BS>(lead ? total - kept : 0, sh);
-    int mx = block_max_int<BS>(lead ? kept : 0, sh);
-    if (threadIdx.x == 0) {
-        if (tot) atomicAdd(&s.st->nbr_total, (unsigned long long)tot);
-        if (ov) { atomicAdd(&s.st->overflow, ov); atomicOr(&s.st->status, 8u); }
-        if (mx) atomicMax(&s.st->max_nbrs, mx);
-    }
-}
-
 __global__ void k_boundary_keys(const float4* bpos, int nb, GridGeom g, int* keys) {
     int i = blockIdx.x * NT + threadIdx.x;
     if (i >= nb) return;
@@ -629,15 +523,8 @@ void preload_build_kernels() {
 
 void launch_build(const DevScene& s, const GridGeom& g, const SolverConst& c, int mode, int n_max, cudaStream_t st,
                   int bs) {
-    if (c.build) {
+    if (c.build == 1 || (c.build == 2 && mode == 0)) {
         launch_warp_build(s, g, c, mode, n_max, st, bs);
-        return;
-    }
-    if (mode == 2 && c.lanes == 4 && c.cap <= LROW - 4) {
-        // small scenes: 4 threads per particle (sizes measured: 27 k particles,
-        // 54 -> 35 us; 8 threads per particle 40 us)
-        const int nb = (int)(((long long)(n_max > 0 ? n_max : 1) * 4 + 127) / 128);
-        k_build_wc_lanes<4><<<nb, 128, sizeof(int) * LROW * 128, st>>>(s, g, c);
         return;
     }
     if (bs == 64) launch_build_bs<64>(s, g, c, mode, n_max, st);
@@ -646,7 +533,7 @@ void launch_build(const DevScene& s, const GridGeom& g, const SolverConst& c, in
 }
 
 int build_blocks(const SolverConst& c, int n_max, int bs) {
-    if (c.build) return warp_build_blocks(n_max, bs);
+    if (c.build == 1) return warp_build_blocks(n_max, bs);
     return nblk(n_max > 0 ? n_max : 1, bs == 64 || bs == 256 ? bs : 128);
 }
 
