@@ -500,10 +500,32 @@ __device__ __forceinline__ float sqrt_approx(float x) {
     return y;
 }
 
-// ker_spline (surface_field.cpp:235-249), times the particle volume
-__device__ __forceinline__ float sf_spline(const SfParams& P, float r) {
-    const float hr = P.r_h - r;
-    return r < 0.5f * P.r_h ? fmaf(P.p3 * r, r * r, fmaf(P.p2, r * r, P.p1)) : P.p4 * hr * hr * hr;
+// packed FP32 pairs (sm_100's f32x2 operations: each half rounded as its
+// scalar form)
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pair(float lo, float hi) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1,%2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ f32x2 both(float v) { return pair(v, v); }
+__device__ __forceinline__ void split(f32x2 v, float& lo, float& hi) {
+    asm("mov.b64 {%0,%1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
 }
 
 // One CTA per tile, one thread per x-row of 8 nodes; a warp's rows are a patch
@@ -514,9 +536,11 @@ __device__ __forceinline__ float sf_spline(const SfParams& P, float r) {
 // staged with the particle): rows whose minimum lies beyond r_h^2 are left at
 // once, and the nodes of a half-row are evaluated together when one of them is
 // inside.  Bound by the instructions of rows that the ellipsoid only grazes:
-// 46 656 anisotropic particles on 151^3 nodes take 224 us (326 with rows of 16 x 2
+// 46 656 anisotropic particles on 151^3 nodes take 215 us (326 with rows of 16 x 2
 // a warp, every particle of the tile tested by every warp, and the row's
-// interval from the quadratic's roots); 216 000 isotropic ones 437 us (584).
+// interval from the quadratic's roots; 225 with scalar instead of packed FP32
+// arithmetic); 216 000 isotropic ones 417 us (584; 437).  Five or six blocks per
+// SM declared instead of the four that 52 registers leave: 236 and 225 us.
 constexpr int PY = 8, PZ = 4;  // rows of a warp's patch
 __global__ void __launch_bounds__(FT) k_sf_field(SfParams P, const int* tstart, const int* ppart, const float4* rec0,
                                                  const float4* rec1, const float4* rec2, const int4* box_lo,
@@ -579,29 +603,39 @@ __global__ void __launch_bounds__(FT) k_sf_field(SfParams P, const int* tstart, 
                 // min_k r^2 = r_h^2 - disc / |du|^2: the row misses the ellipsoid
                 // (kept when within rounding of touching it)
                 if (disc < -1e-5f * rh2 * du.w) continue;
-                const float B2 = 2.f * B;
+                const f32x2 A2 = both(du.w), B2 = both(2.f * B), C2 = both(C0);
 #pragma unroll
                 for (int half = 0; half < 2; ++half) {
-                    float r2[TX / 2];
+                    f32x2 r2[TX / 4];
                     bool in[TX / 2], any = false;
 #pragma unroll
-                    for (int q = 0; q < TX / 2; ++q) {
-                        const int k = half * (TX / 2) + q;
-                        const float fk = (float)k;
-                        r2[q] = fmaf(fmaf(du.w, fk, B2), fk, C0);
-                        in[q] = r2[q] <= rh2 && k >= xa && k <= xb;
-                        any |= in[q];
+                    for (int q = 0; q < TX / 4; ++q) {
+                        const int k = half * (TX / 2) + 2 * q;
+                        const f32x2 fk = pair((float)k, (float)(k + 1));
+                        r2[q] = fma2(fma2(A2, fk, B2), fk, C2);
+                        float lo_, hi_;
+                        split(r2[q], lo_, hi_);
+                        in[2 * q] = lo_ <= rh2 && k >= xa && k <= xb;
+                        in[2 * q + 1] = hi_ <= rh2 && k + 1 >= xa && k + 1 <= xb;
+                        any |= in[2 * q] || in[2 * q + 1];
                     }
                     if (!any) continue;
 #pragma unroll
-                    for (int q = 0; q < TX / 2; ++q) {
+                    for (int q = 0; q < TX / 4; ++q) {
                         // ker_spline (surface_field.cpp:235-249), times the particle
                         // volume: p1 + r^2 (p2 + p3 r) inside h/2, p4 (h - r)^3 beyond
-                        const float r = sqrt_approx(r2[q]);
-                        const float hr = rh - r;
-                        const float w = r < hh ? fmaf(fmaf(P.p3, r, P.p2), r2[q], P.p1) : (P.p4 * hr) * (hr * hr);
-                        const float sum = fmaf(c.w, w, acc[half * (TX / 2) + q]);
-                        if (in[q]) acc[half * (TX / 2) + q] = sum;
+                        float ra, rb;
+                        split(r2[q], ra, rb);
+                        ra = sqrt_approx(ra);
+                        rb = sqrt_approx(rb);
+                        const f32x2 r = pair(ra, rb), hr = sub2(both(rh), r);
+                        float na, nb, fa, fb;
+                        split(fma2(fma2(both(P.p3), r, both(P.p2)), r2[q], both(P.p1)), na, nb);
+                        split(mul2(mul2(both(P.p4), hr), mul2(hr, hr)), fa, fb);
+                        float* a = acc + half * (TX / 2) + 2 * q;
+                        split(fma2(both(c.w), pair(ra < hh ? na : fa, rb < hh ? nb : fb), pair(a[0], a[1])), na, nb);
+                        if (in[2 * q]) a[0] = na;
+                        if (in[2 * q + 1]) a[1] = nb;
                     }
                 }
             }
