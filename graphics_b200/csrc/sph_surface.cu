@@ -1181,7 +1181,7 @@ long long sphgpu_surface_mesh(sphgpu_surface_t s, float iso, int ref_rows, float
     SCK(cudaStreamSynchronize(st));
     const long long total = (long long)last_off + last_n;  // < 2^31: 5 triangles per cube at most
     s->ntris = total;
-    if (!out || total == 0) return total;
+    if (total == 0) return 0;
     if (total > s->tricap) {
         if (salloc(s, &s->tris, 9 * (size_t)total)) return SPHGPU_ENOMEM;
         s->tricap = total;
@@ -1190,7 +1190,8 @@ long long sphgpu_surface_mesh(sphgpu_surface_t s, float iso, int ref_rows, float
     k_mc_emit<<<(int)nblocks, MCB, 0, st>>>(M, s->field, ngroups, gpr, s->cases, s->ntri, s->toff, s->tris);
     SCK(cudaGetLastError());
     SCK(cudaStreamSynchronize(st));
-    SCK(copy_sync(out, s->tris, sizeof(float) * 9 * (size_t)std::min(total, max_tris), cudaMemcpyDeviceToHost));
+    if (out)
+        SCK(copy_sync(out, s->tris, sizeof(float) * 9 * (size_t)std::min(total, max_tris), cudaMemcpyDeviceToHost));
     return total;
 }
 
