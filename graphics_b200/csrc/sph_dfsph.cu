@@ -17,7 +17,7 @@
 // per neighbour: {position, loop velocity} (32 B) in the A sweeps and
 // (x, y, z, kappa/rho) (16 B) in the B sweeps.  Per-particle arithmetic is
 // FP32; the convergence sums are FP64 block partials reduced in a fixed order
-// by the last block, so results are run-to-run deterministic.
+// by the B sweep's first block, so results are run-to-run deterministic.
 //
 // Loop control: k_*_b decides whether another iteration runs.  Inside a CUDA
 // graph the loop is a conditional WHILE node and the decision is written with

@@ -27,7 +27,7 @@
 // updates the loop velocity with both:
 //   v_i -= dt/m_i sum_j gradW_ij (V_i^2 V_j kappa_i/gamma_i + V_j^2 V_i kappa_j/gamma_j).
 // Per-particle arithmetic is FP32; the error sums are FP64 block partials
-// reduced in a fixed order by the last block.  Phases are solved in turn,
+// reduced in a fixed order by sweep B's first block.  Phases are solved in turn,
 // as the reference does; the loop velocities of the other phases are the
 // carried ones (the reference keeps advectionVelocity in the particle).
 //
@@ -356,9 +356,9 @@ __global__ void __launch_bounds__(BS, 1024 / BS) k_iv_sweep_a(DevScene s, Solver
 // Sweep B's first block, which takes no particles: the error sum of sweep A's
 // `parts` blocks and the loop decision (as DFSPH's b_decide: a last block of
 // sweep A that waited for the others ended each with some 3 us of fence,
-// atomic and loads;
-// 64 k particles, event-timed: 18.2 -> 14.7 us a sweep A, sweep B 14.8 as before).  Continue while the error is above the goal
-// or fewer than min_it iterations ran, and stop once the count exceeds max_it
+// atomic and loads; 64 k particles, event-timed: 18.2 -> 14.7 us a sweep A,
+// sweep B 14.8 as before).  Continue while the error is above the goal or
+// fewer than min_it iterations ran, and stop once the count exceeds max_it
 // (the reference breaks when it > max, IISph.cpp:558,1234).
 template <int BS, int DIV>
 __device__ __forceinline__ void iv_decide(const DevScene& s, int parts, double goal, int min_it, int max_it,

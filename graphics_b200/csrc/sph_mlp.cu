@@ -12,10 +12,11 @@
 // starts, and the gain is counted in iterations.
 //
 // GEMMs run on the tensor cores with mma.sync.m16n8k16 (BF16 operands, FP32
-// accumulation): a 128-row tile per 4-warp block, each warp owning 32 rows.
-// Training (forward + backward of a mini-batch, FP32 gradient atomics) and
-// Adam (FP32 master weights, BF16 copies for the GEMMs) are separate
-// kernels; inference is fused into the per-particle feature sweep.
+// accumulation): 128-row tiles, in training (forward + backward of a
+// mini-batch, one gradient slot per tile) by 16 warps, in prediction by four
+// with 32 rows each.  A second kernel sums the slots in tile order and applies
+// Adam (FP32 master weights, BF16 copies for the GEMMs); inference is fused
+// into the per-particle feature sweep.
 #include <cuda_bf16.h>
 
 #include "sph_kernels.cuh"
