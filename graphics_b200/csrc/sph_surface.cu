@@ -803,7 +803,7 @@ struct sphgpu_surface {
     int pcap = 0;
     float* xyz = nullptr;  // host positions staged on the device
     double* mom = nullptr;  // 6 per particle
-    float4 *pos = nullptr, *spos = nullptr, *rec0 = nullptr, *rec1 = nullptr, *rec2 = nullptr;
+    float4 *pos = nullptr, *rec0 = nullptr, *rec1 = nullptr, *rec2 = nullptr;
     int4 *blo = nullptr, *bhi = nullptr;
     int *key = nullptr, *slot = nullptr, *tmp = nullptr, *npair = nullptr, *poff = nullptr;
     int* pcnt = nullptr;    // neighbour-grid cells + 2
@@ -879,7 +879,7 @@ int ensure_particles(sphgpu_surface* s, int n) {
     const int cap = std::max(n, 2 * s->pcap);
     int r = salloc(s, &s->pos, cap) | salloc(s, &s->rec0, cap) | salloc(s, &s->rec1, cap) | salloc(s, &s->rec2, cap) |
             salloc(s, &s->blo, cap) | salloc(s, &s->bhi, cap) | salloc(s, &s->key, cap) | salloc(s, &s->slot, cap) |
-            salloc(s, &s->tmp, cap) | salloc(s, &s->spos, cap) | salloc(s, &s->mom, 6 * (size_t)cap) | salloc(s, &s->npair, (size_t)cap + 1) |
+            salloc(s, &s->tmp, cap) | salloc(s, &s->mom, 6 * (size_t)cap) | salloc(s, &s->npair, (size_t)cap + 1) |
             salloc(s, &s->poff, (size_t)cap + 1) | salloc(s, &s->xyz, 3 * (size_t)cap);
     if (r) return SPHGPU_ENOMEM;
     s->pcap = cap;
@@ -898,6 +898,7 @@ int run_field(sphgpu_surface* s, int n, int aniso) {
     const int pcells = P.pnum[0] * P.pnum[1] * P.pnum[2];
     // neighbour grid (anisotropic kernels only)
     if (aniso && n > 0) {
+        float4* const spos = s->rec1;  // positions in cell order until k_sf_kernel writes the record
         SCK(cudaMemsetAsync(s->pcnt, 0, sizeof(int) * ((size_t)pcells + 2), st));
         SCK(cudaMemsetAsync(s->bad, 0, sizeof(int), st));
         s->kernels += 4;
@@ -907,8 +908,8 @@ int run_field(sphgpu_surface* s, int n, int aniso) {
         if (int r = ensure_tmp(s, b)) return r;
         cub::DeviceScan::ExclusiveSum(s->tmpbuf, b, s->pcnt, s->pstart, pcells + 2, st);
         k_sf_scatter<<<nblk(n, 256), 256, 0, st>>>(s->key, s->slot, s->pstart, n, s->tmp);
-        k_sf_rank<<<nblk(n, 256), 256, 0, st>>>(s->key, s->pstart, s->tmp, s->pos, n, s->spos);
-        k_sf_moments<<<nblk(n, MNT / ML), MNT, 0, st>>>(P, s->spos, n, s->pstart, s->rec0, s->npair, s->mom);
+        k_sf_rank<<<nblk(n, 256), 256, 0, st>>>(s->key, s->pstart, s->tmp, s->pos, n, spos);
+        k_sf_moments<<<nblk(n, MNT / ML), MNT, 0, st>>>(P, spos, n, s->pstart, s->rec0, s->npair, s->mom);
     }
     s->kernels += n > 0;
     if (n > 0)
@@ -1045,7 +1046,7 @@ int sphgpu_surface_create(const double* mn, const double* mx, double r_p, double
 int sphgpu_surface_destroy(sphgpu_surface_t s) {
     if (!s) return SPHGPU_EINVAL;
     cudaSetDevice(s->device);
-    void* ptrs[] = {s->field, s->xyz, s->pos, s->rec0, s->rec1, s->rec2, s->blo, s->bhi, s->key, s->slot, s->tmp, s->spos, s->mom,
+    void* ptrs[] = {s->field, s->xyz, s->pos, s->rec0, s->rec1, s->rec2, s->blo, s->bhi, s->key, s->slot, s->tmp, s->mom,
                     s->npair, s->poff, s->pcnt, s->pstart, s->bad, s->ptile, s->ppart, s->ptile_s, s->ppart_s,
                     s->tstart, s->ntri, s->toff, s->cases, s->tris, s->coords, s->tmpbuf};
     for (void* p : ptrs)
