@@ -238,7 +238,7 @@ __device__ __forceinline__ float iv_div_sum(const DevScene& s, const SolverConst
     const float Vf = c.iv_V;
     float acc = 0.f;
     const unsigned long long polL = l2_policy(c.l2pol & 3);  // lists stream through L2
-    int4 nxt = ng ? ell_group_pol(s.nbr, stride, p, 0, polL) : make_int4(0, 0, 0, 0);
+    int4 nxt = ell_group_pol(s.nbr, stride, p, 0, polL);
     for (int gi = 0; gi < ng; ++gi) {
         const int4 cur = nxt;
         if (gi + 1 < ng) nxt = ell_group_pol(s.nbr, stride, p, gi + 1, polL);
@@ -410,7 +410,7 @@ __global__ void __launch_bounds__(BS) k_iv_sweep_b(DevScene s, SolverConst c, in
             const int ng = (cnt + 3) >> 2;
             const size_t stride = (size_t)c.stride;
             const unsigned long long polL = l2_policy(c.l2pol & 3);  // lists stream through L2
-            int4 nxt = ng ? ell_group_pol(s.nbr, stride, p, 0, polL) : make_int4(0, 0, 0, 0);
+            int4 nxt = ell_group_pol(s.nbr, stride, p, 0, polL);
             for (int gi = 0; gi < ng; ++gi) {
                 const int4 cur = nxt;
                 if (gi + 1 < ng) nxt = ell_group_pol(s.nbr, stride, p, gi + 1, polL);

@@ -232,15 +232,16 @@ __device__ __forceinline__ float div_term(const SolverConst& c, float4 pa, float
     return fmaf(t, m, acc);
 }
 
-// Walks an ELL list of cnt entries by one thread, four at a time: the next
-// group's load is issued before ld(t, entry), t < 4, issues the current
+// Walks an ELL list of cnt entries by one thread, four at a time: the first
+// group's load does not wait for the count (a cap of at least 1 gives every
+// slot one), the next group's load is issued before ld(t, entry), t < 4, issues the current
 // one's gathers (entries past the count: `self`), then use(t, entry) takes
 // the entries of the list in order.
 template <class Ld, class Use>
 __device__ __forceinline__ void walk4(const int* list, size_t stride, int p, int cnt, unsigned self,
                                       unsigned long long pol, Ld&& ld, Use&& use) {
     const int ng = (cnt + 3) >> 2;
-    int4 nxt = ng ? ell_group_pol(list, stride, p, 0, pol) : make_int4(0, 0, 0, 0);
+    int4 nxt = ell_group_pol(list, stride, p, 0, pol);
     for (int gi = 0; gi < ng; ++gi) {
         const int4 cur = nxt;
         if (gi + 1 < ng) nxt = ell_group_pol(list, stride, p, gi + 1, pol);

@@ -633,7 +633,7 @@ __device__ __forceinline__ void ws_features(const DevScene& s, const SolverConst
     // particle's own record and are masked out
     const int ng = (cnt + 3) >> 2;
     const unsigned long long polL = l2_policy(c.l2pol & 3);  // lists stream through L2
-    int4 nxt = ng ? ell_group_pol(s.nbr, stride, p, 0, polL) : make_int4(0, 0, 0, 0);
+    int4 nxt = ell_group_pol(s.nbr, stride, p, 0, polL);
     for (int gi = 0; gi < ng; ++gi) {
         const int4 cur = nxt;
         if (gi + 1 < ng) nxt = ell_group_pol(s.nbr, stride, p, gi + 1, polL);

@@ -175,7 +175,7 @@ __global__ void __launch_bounds__(NT) k_pci_density(DevScene s, SolverConst c, f
         const unsigned long long polL = l2_policy(c.l2pol & 3);  // lists stream through L2
         // four list entries per 16-byte load, the next group's issued before
         // the current group's gathers; the sum stays in list order
-        int4 nxt = ng ? ell_group_pol(s.nbr, stride, p, 0, polL) : make_int4(0, 0, 0, 0);
+        int4 nxt = ell_group_pol(s.nbr, stride, p, 0, polL);
         for (int gi = 0; gi < ng; ++gi) {
             const int4 cur = nxt;
             if (gi + 1 < ng) nxt = ell_group_pol(s.nbr, stride, p, gi + 1, polL);
@@ -241,7 +241,7 @@ __global__ void __launch_bounds__(NT, 9) k_pci_pressure(DevScene s, SolverConst 
         // one 32-byte record per fluid neighbour ({position, (rho, p)}, written
         // by this iteration's density sweep); boundary neighbours: position
         // and volume
-        int4 nxt = ng ? ell_group_pol(s.nbr, stride, p, 0, polL) : make_int4(0, 0, 0, 0);
+        int4 nxt = ell_group_pol(s.nbr, stride, p, 0, polL);
         for (int gi = 0; gi < ng; ++gi) {
             const int4 cur = nxt;
             if (gi + 1 < ng) nxt = ell_group_pol(s.nbr, stride, p, gi + 1, polL);

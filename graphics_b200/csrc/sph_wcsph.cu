@@ -226,7 +226,7 @@ __global__ void __launch_bounds__(NT) k_wc_force(DevScene s, SolverConst c) {
             const WcPlain w = wc_plain(o, c);
             const unsigned long long polL = l2_policy(c.l2pol & 3);  // lists stream through L2
             const int ng = (cnt + 3) >> 2;
-            int4 nxt = ng ? ell_group_pol(s.nbr, stride, p, 0, polL) : make_int4(0, 0, 0, 0);
+            int4 nxt = ell_group_pol(s.nbr, stride, p, 0, polL);
             for (int gi = 0; gi < ng; ++gi) {
                 const int4 cur = nxt;
                 if (gi + 1 < ng) nxt = ell_group_pol(s.nbr, stride, p, gi + 1, polL);
