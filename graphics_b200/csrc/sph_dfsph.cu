@@ -428,9 +428,10 @@ constexpr int LROWS = 52;  // entries per particle's row (cap <= 48): rows start
 
 // The lane's first entries, loaded before the particle's count (and whether it
 // is a particle at all) is known: one latency less in the chain.  The same for
-// the first list group of the one-thread sweeps.  An iteration of the density
-// loop, before / now: 1 k particles 14.2 / 11.7 us, 8 k 14.9 / 12.7, 69 k 22.1 /
-// 20.2, 343 k 66.7 / 65.4.
+// the first list group of the one-thread sweeps.  Event-timed before / now: A 1 k
+// particles 11.4 / 10.5 us, 8 k 11.8 / 11.0, B 1 k 9.0 / 8.6, 8 k 10.6 / 8.8; one
+// thread per particle at 69 k and above as before (16.5, 12.7).  The count
+// loaded as early too: no further gain.
 constexpr int LAHEAD = 4;
 __device__ __forceinline__ void lane_ahead(const DevScene& s, const SolverConst& c, int p, int t,
                                            unsigned e[LAHEAD]) {
