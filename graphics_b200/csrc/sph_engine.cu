@@ -18,6 +18,7 @@
 #include <vector>
 
 #include "../../include/sphgpu.h"
+#include "sph_batch.cuh"
 #include "sph_kernels.cuh"
 #include "sph_mlp.cuh"
 #include "sph_sync.cuh"
@@ -361,6 +362,22 @@ int dalloc(sphgpu_scene* h, T** p, size_t n) {
     return 0;
 }
 
+// Per-block FP64 sums (DevScene::partial) of the largest grid that any kernel
+// writing them can have: every block size, list build and thread count per
+// particle that the rules, the autotuner or a debug knob choose, the chunks of
+// a batch (one at least per scene), and two sums a block (PCISPH, IISPH_M).
+size_t partial_slots(const sphgpu_scene* h) {
+    SolverConst c = h->c;
+    int m = batch_chunks(h->cap, h->nscenes);
+    for (int bs : {64, 128, 256})
+        for (int v : {0, 1}) {
+            c.lanes_a = v ? 4 : 1;
+            c.build = v;
+            m = std::max({m, df_a_blocks(c, h->cap, bs), build_blocks(c, h->cap, bs)});
+        }
+    return 2 * (size_t)m;
+}
+
 int alloc_scene(sphgpu_scene* h) {
     const int n = h->cap;
     DevScene& d = h->d;
@@ -384,7 +401,7 @@ int alloc_scene(sphgpu_scene* h) {
     r |= dalloc(h, &d.bcell_start, (size_t)h->g.nkeys + 1);
     r |= dalloc(h, &d.nbr, (size_t)h->stride * ((h->ncap + 3) / 4) * 4);
     r |= dalloc(h, &d.ncount, n);
-    r |= dalloc(h, &d.partial, (size_t)n / 64 + 4096);
+    r |= dalloc(h, &d.partial, partial_slots(h));
     r |= dalloc(h, &d.st, 1);
     if (r) return SPHGPU_ENOMEM;
     d.cap_fluid = n;
