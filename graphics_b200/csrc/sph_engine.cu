@@ -129,7 +129,7 @@ struct sphgpu_scene {
     // priority, so the records the sweeps gather stay resident (measured at
     // 1 M: density sweeps A/B 135/74 -> 129/72 us; records evict-last: no gain)
     int l2pol = 1;
-    // the list build (SolverConst::build): -1 by size, else 0 or 1 (debug knob "build")
+    // the list build (SolverConst::build): -1 by size, else 0, 1 or 2 (debug knob "build")
     int build = -1;
     int sweep_lanes = 0;  // SolverConst::lanes_a, lanes_b: 0 by size, 1 or 4 (debug knob "sweep_lanes")
     int scan_max = SCAN_MAX;  // cell keys scanned by one block (debug knob "scan": 0 CUB, else one block)
@@ -308,7 +308,7 @@ void fill_solver_const(sphgpu_scene* h) {
     c.th_bt = P.th_bt;
     c.cap = h->ncap;
     c.build = h->ncap > 48 ? 0
-              : h->build >= 0 ? h->build != 0
+              : h->build >= 0 ? h->build
                               : (h->cap <= WARP_BUILD_MAX ? 1 : (h->cap <= WARP_LISTS_MAX ? 2 : 0));
     c.stride = h->stride;
     c.l2pol = h->l2pol;
@@ -2939,7 +2939,7 @@ int sphgpu_get_solid_force(sphgpu_t h, int solid_id, double force[3], double tor
 //   l2_policy              L2 eviction priorities of the sweeps' list and record loads
 //   fuse_div               DFSPH: the list build runs the divergence loop's first sweep A
 //   sweep_lanes            threads per particle of the DFSPH sweeps (0 by size, 1, 4)
-//   build                  list build (-1 by size, 0 a thread per particle, 1 a warp for a few)
+//   build                  list build (SolverConst::build: -1 by size, 0, 1, 2)
 //   scan                   cell-count scan: 0 CUB over the chip, else one block
 //   fuse_ws                warm start: feature gather and network in one kernel
 //   speculative_host_step  sphgpu_step_host runs part 1 while checking its inputs
@@ -2958,6 +2958,7 @@ int sphgpu_debug_set(sphgpu_t h, const char* key, int value) {
         return 0;
     }
     if (k == "build") {
+        if (value < -1 || value > 2) return SPHGPU_EINVAL;
         h->build = value;
         fill_solver_const(h);
         invalidate_graphs(h);

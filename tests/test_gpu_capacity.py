@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 
 from graphics_b200.scene import dam_break, rayleigh_taylor
-from graphics_b200.sph import GpuBatch, GpuScene, params_for_scene
+from graphics_b200.sph import GpuBatch, GpuScene, SphGpuError, params_for_scene
 
 pytestmark = pytest.mark.gpu
 
@@ -59,6 +59,21 @@ def test_forced_kernels_in_a_large_handle(knobs):
                                         ("iisph", 65_537)])
 def test_capacity_does_not_change_results(solver, cap):
     _same(_run(solver), _run(solver, cap))
+
+
+# lists by warps and the sums by threads: what handles of 65 537 to 262 144 particles run
+@pytest.mark.parametrize("solver", sorted(KW))
+def test_lists_alone_by_warps(solver):
+    _same(_run(solver, knobs=[("build", 0)]), _run(solver, knobs=[("build", 2)]))
+
+
+def test_unknown_list_builds_are_refused():
+    sc = _scene("dfsph", (2, 2, 2))
+    g = GpuScene(params_for_scene(sc, **DF), sc.n_fluid)
+    for v in (-2, 3):
+        with pytest.raises(SphGpuError):
+            g.debug_set("build", v)
+    g.close()
 
 
 def test_a_batch_of_more_scenes_than_blocks():
