@@ -106,10 +106,7 @@ __device__ __forceinline__ double sums_finish(const DevScene& s, const SolverCon
         float pr = c.wc_B * (powf(density / rho0, c.wc_gamma) - 1.f);
         if (pr < 0.f) pr = 0.f;
         s.kr[p] = pr;
-        // the force pass's record
-        const float4 v = s.vel[p];
-        s.prv[2 * p] = make_float4(pa.x, pa.y, pa.z, density);
-        s.prv[2 * p + 1] = make_float4(v.x, v.y, v.z, pr / (density * density));
+        wc_record(s, p, pa, s.vel[p], density, pr);
         return 0.0;
     }
     s.prv[2 * p] = make_float4(pa.x, pa.y, pa.z, density);

@@ -2278,6 +2278,7 @@ int sphgpu_stage(sphgpu_t h, const char* name, SphStepStats* stats) {
         if (h->in_staging) { h->err = "run neighbourSearch first"; return SPHGPU_EINVAL; }
         const bool surf = h->P.th_h != 0.f || h->P.th_r != 0.f || h->P.th_bt != 0.f;
         if (surf) launch_wc_normal(d, h->c, h->cap, st);
+        launch_wc_records(d, h->cap, st);
         launch_wc_force(d, h->c, h->cap, st, surf, h->c.lanes);
         h->ep_acc = h->sorts;
         h->in_staging = true;

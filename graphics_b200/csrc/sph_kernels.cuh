@@ -182,6 +182,12 @@ __device__ __forceinline__ void stats_step_begin(DevStats* st) {
     st->err_div = 0;
 }
 
+// the record of WCSPH's plain force pass: {(x, y, z, rho), (v, p/rho^2)}
+__device__ __forceinline__ void wc_record(const DevScene& s, int p, float4 x, float4 v, float rho, float pr) {
+    s.prv[2 * p] = make_float4(x.x, x.y, x.z, rho);
+    s.prv[2 * p + 1] = make_float4(v.x, v.y, v.z, pr / (rho * rho));
+}
+
 // step length of the particle's scene
 __device__ __forceinline__ float dt_of(const DevScene& s, float4 pa) {
     return s.nscenes > 1 ? s.b.dt[scene_of(pa)] : *s.dt;
@@ -331,6 +337,9 @@ void launch_batch_count(const DevScene& s, int nscenes, cudaStream_t st);
 void launch_wc_force(const DevScene& s, const SolverConst& c, int n_max, cudaStream_t st, bool surf = false,
                      int lanes = 1);
 void launch_wc_normal(const DevScene& s, const SolverConst& c, int n_max, cudaStream_t st);
+// the force pass's records again from positions, velocities, densities and
+// pressures (the list build writes them; a stage may follow changed fields)
+void launch_wc_records(const DevScene& s, int n_max, cudaStream_t st);
 
 // ---- PCISPH / IISPH_M (sph_pci_ii.cu) ----
 void launch_pci_force_except(const DevScene& s, const SolverConst& c, int n_max, cudaStream_t st);

@@ -301,8 +301,15 @@ __global__ void __launch_bounds__(NT) k_wc_force_lanes(DevScene s, SolverConst c
         if (zero) atomicAdd(&s.st->zero_dis, zero);
     }
 }
+__global__ void __launch_bounds__(NT) k_wc_records(DevScene s) {
+    const int p = blockIdx.x * NT + threadIdx.x;
+    if (p < s.st->n_active) wc_record(s, p, s.pos[p], s.vel[p], s.rho[p], s.kr[p]);
+}
 }  // namespace
 
+void launch_wc_records(const DevScene& s, int n_max, cudaStream_t st) {
+    k_wc_records<<<(n_max + NT - 1) / NT, NT, 0, st>>>(s);
+}
 void launch_wc_force(const DevScene& s, const SolverConst& c, int n_max, cudaStream_t st, bool surf, int lanes) {
     if (lanes == 4) {
         const int nb = (int)(((long long)n_max * 4 + NT - 1) / NT);

@@ -1,0 +1,37 @@
+"""Solver stages after fields that the caller has set between them (GPU)."""
+import numpy as np
+import pytest
+
+from graphics_b200.scene import dam_break
+from graphics_b200.sph import GpuScene, params_for_scene
+
+pytestmark = pytest.mark.gpu
+
+
+# WCSPH's plain force pass reads a record per neighbour, which the list build
+# writes; the general pass (a second fluid: one particle out of reach in the
+# far corner) reads the fields themselves
+@pytest.mark.parametrize("lanes", [1, 4])
+def test_wcsph_forces_after_set_density(lanes):
+    r, counts = 0.0125, (12, 11, 13)
+    sc = dam_break(counts, r, tuple(2 * r * (k + 3) for k in counts), seed=4)
+    rng = np.random.default_rng(4)
+    sc.fluid_vel = rng.normal(0, 0.2, sc.fluid_pos.shape).astype(np.float32)
+    factor = rng.uniform(0.8, 1.25, sc.n_fluid + 1).astype(np.float32)
+    acc = []
+    for far in (0, 1):
+        g = GpuScene(params_for_scene(sc, dt=2.5e-4, soundSpeed_cs=18.0, boundary_visc=0.03), sc.n_fluid + 1)
+        g.debug_set("wc_lanes", lanes)
+        g.set_boundary(sc.boundary_pos)
+        g.add_fluid(sc.fluid_pos, sc.fluid_vel, visc_alpha=0.05)
+        if far:
+            g.add_fluid(np.array([[(k + 2.5) * sc.d for k in counts]], np.float32), rho0=2000.0, visc_alpha=0.05)
+        g.stage("wc_computePressure")
+        before = g.get("density")
+        g.set("density", before * factor[:len(before)])
+        np.testing.assert_array_equal(g.get("density"), before * factor[:len(before)])
+        g.stage("wc_computeForce")
+        acc.append(g.get("acceleration")[:sc.n_fluid])
+        g.close()
+    # some 50 terms, each a few ulp of the largest, in either pass: 50 * 4 * 2^-24
+    assert np.abs(acc[0] - acc[1]).max() <= 50 * 4 * 2.0 ** -24 * np.abs(acc[0]).max()
