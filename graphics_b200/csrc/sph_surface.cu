@@ -855,12 +855,16 @@ int ensure_table(sphgpu_surface* s) {
     return 0;
 }
 
+// The buffer anew with room for n.  Where a capacity goes with it, the caller
+// sets that to 0 first and to its value when all of its buffers are there: after
+// a failure a smaller input allocates again.
 template <class T>
 int salloc(sphgpu_surface* s, T** p, size_t n) {
     if (*p) cudaFree(*p);
     *p = nullptr;
     cudaError_t e = cudaMalloc((void**)p, std::max<size_t>(n, 1) * sizeof(T));
     if (e != cudaSuccess) {
+        cudaGetLastError();  // reported here, not by a later call's check
         s->err = std::string("cudaMalloc: ") + cudaGetErrorString(e);
         return SPHGPU_ENOMEM;
     }
@@ -869,19 +873,19 @@ int salloc(sphgpu_surface* s, T** p, size_t n) {
 
 int ensure_tmp(sphgpu_surface* s, size_t bytes) {
     if (bytes <= s->tmpbytes) return 0;
-    if (s->tmpbuf) cudaFree(s->tmpbuf);
-    s->tmpbuf = nullptr;
-    if (cudaMalloc(&s->tmpbuf, bytes + 256) != cudaSuccess) {
-        s->err = "cudaMalloc (scratch) failed";
-        return SPHGPU_ENOMEM;
-    }
+    s->tmpbytes = 0;
+    char* p = (char*)s->tmpbuf;
+    const int r = salloc(s, &p, bytes + 256);
+    s->tmpbuf = p;
+    if (r) return r;
     s->tmpbytes = bytes;
     return 0;
 }
 
 int ensure_particles(sphgpu_surface* s, int n) {
     if (n <= s->pcap) return 0;
-    const int cap = std::max(n, 2 * s->pcap);
+    const int cap = (int)std::min<long long>(std::max<long long>(n, 2ll * s->pcap), 0x7fffffffll);
+    s->pcap = 0;
     int r = salloc(s, &s->pos, cap) | salloc(s, &s->rec0, cap) | salloc(s, &s->rec1, cap) | salloc(s, &s->rec2, cap) |
             salloc(s, &s->blo, cap) | salloc(s, &s->bhi, cap) | salloc(s, &s->key, cap) | salloc(s, &s->slot, cap) |
             salloc(s, &s->tmp, cap) | salloc(s, &s->mom, 6 * (size_t)cap) | salloc(s, &s->npair, (size_t)cap + 1) |
@@ -937,6 +941,7 @@ int run_field(sphgpu_surface* s, int n, int aniso) {
     }
     if (npairs > s->paircap) {
         const long long cap = std::max(npairs, 2 * s->paircap);
+        s->paircap = 0;
         if (salloc(s, &s->ptile, cap) | salloc(s, &s->ppart, cap) | salloc(s, &s->ptile_s, cap) |
             salloc(s, &s->ppart_s, cap))
             return SPHGPU_ENOMEM;
@@ -1130,10 +1135,12 @@ long long sphgpu_surface_mesh(sphgpu_surface_t s, float iso, int ref_rows, float
     const long long ngroups = (long long)gpr * (g[1] - 1) * (g[2] - 1);
     const long long nblocks = (ngroups + MCB - 1) / MCB;
     if (nblocks > s->cubecap) {
+        s->cubecap = 0;
         if (salloc(s, &s->ntri, (size_t)nblocks) || salloc(s, &s->toff, (size_t)nblocks)) return SPHGPU_ENOMEM;
         s->cubecap = nblocks;
     }
     if (ncubes > s->casecap) {
+        s->casecap = 0;
         if (salloc(s, &s->cases, (size_t)ncubes)) return SPHGPU_ENOMEM;
         s->casecap = ncubes;
     }
@@ -1189,6 +1196,7 @@ long long sphgpu_surface_mesh(sphgpu_surface_t s, float iso, int ref_rows, float
     s->ntris = total;
     if (total == 0) return 0;
     if (total > s->tricap) {
+        s->tricap = 0;
         if (salloc(s, &s->tris, 9 * (size_t)total)) return SPHGPU_ENOMEM;
         s->tricap = total;
     }

@@ -1,0 +1,78 @@
+"""The surface handle's growing buffers (GPU): a call that found no memory
+leaves a handle that works on."""
+import numpy as np
+import pytest
+
+from graphics_b200 import _lib
+from graphics_b200.sph import SphGpuError
+
+pytestmark = pytest.mark.gpu
+
+
+class _Full:
+    """All of the device's free memory but some 64 MB, while it lasts."""
+
+    def __enter__(self):
+        import torch
+        torch.cuda.synchronize()
+        self.held = []
+        left = torch.cuda.mem_get_info()[0] - (64 << 20)
+        while left >= 1 << 20:
+            try:
+                self.held.append(torch.empty(left, dtype=torch.uint8, device="cuda"))
+                left = torch.cuda.mem_get_info()[0] - (64 << 20)
+            except torch.cuda.OutOfMemoryError:
+                left //= 2
+
+    def __exit__(self, *a):
+        import torch
+        self.held.clear()
+        torch.cuda.empty_cache()
+
+
+def _handle(box=0.2):
+    from graphics_b200.surface import surface_field
+    sf = surface_field()
+    sf.surface_setup([0.0] * 3, [box] * 3, 0.01, 0.02, 0.0025)
+    return sf
+
+
+@pytest.mark.parametrize("aniso", [0, 1])
+def test_field_after_no_memory_for_particles(aniso):
+    import torch
+    rng = np.random.default_rng(1)
+    many = torch.rand((4_000_000, 3), device="cuda") * 0.2
+    pos = rng.uniform(0, 0.2, (3000, 3)).astype(np.float32)
+    fresh, sf = _handle(), _handle()
+    out = []
+    for h in (fresh, sf):
+        field = h.surface_aniso if aniso else h.surface_isotro
+        assert field(pos) == 0  # the buffers hold 3000
+        if h is sf:
+            with _Full():
+                with pytest.raises(SphGpuError) as e:
+                    field(many.data_ptr(), on_device=True, n=len(many))
+            assert e.value.code == _lib.ENOMEM
+        assert field(pos[:2000]) == 0
+        out.append(h.get_field())
+    np.testing.assert_array_equal(*out)
+    fresh.close()
+    sf.close()
+
+
+def test_mesh_after_no_memory_for_triangles():
+    rng = np.random.default_rng(2)
+    sf = _handle(0.5)
+    num = np.asarray(sf.grid_num)
+    f = rng.uniform(0, 1, tuple(num[::-1])).astype(np.float32)
+    few = np.where(np.arange(f.shape[0])[:, None, None] < 3, f, np.float32(2.0))
+    sf.set_field(few)
+    want = sf.mesh(0.5)
+    sf.set_field(f)  # some 2.5 triangles of 36 bytes per cube: over 600 MB
+    with _Full():
+        with pytest.raises(SphGpuError) as e:
+            sf.mesh(0.5)
+    assert e.value.code == _lib.ENOMEM
+    sf.set_field(few)
+    np.testing.assert_array_equal(sf.mesh(0.5), want)
+    sf.close()
