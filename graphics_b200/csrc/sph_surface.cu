@@ -728,7 +728,7 @@ __global__ void __launch_bounds__(MCB) k_mc_count(McParams M, const float* f, lo
 constexpr unsigned long long kEdgeA = 0x321076543210ull;  // kEdge[e][0], 4 bits each
 constexpr unsigned long long kEdgeB = 0x765447650321ull;  // kEdge[e][1]
 __global__ void __launch_bounds__(MCB) k_mc_emit(McParams M, const float* f, long long ngroups, int gpr,
-                                                 const unsigned char* cases, const int* bcount, const int* boff,
+                                                 const unsigned char* cases, const int* bcount, const long long* boff,
                                                  float* out) {
     // most blocks of cubes hold no surface: the whole block leaves at once
     const int total = bcount[blockIdx.x];
@@ -760,7 +760,7 @@ __global__ void __launch_bounds__(MCB) k_mc_emit(McParams M, const float* f, lon
             for (int t = 0; t < nc; ++t) list[at++] = (unsigned short)(threadIdx.x * 32 + (x - x0) * 8 + t);
         }
     __syncthreads();
-    float* o = out + 9 * (long long)boff[blockIdx.x];
+    float* o = out + 9 * boff[blockIdx.x];
     const long long plane = (long long)M.res[0] * M.res[1];
     for (int i = threadIdx.x; i < 3 * total; i += MCB) {
         const int e = list[i / 3];
@@ -821,7 +821,7 @@ struct sphgpu_surface {
     // marching cubes
     long long cubecap = 0, tricap = 0, ntris = 0;
     int* ntri = nullptr;  // triangles per block of MCB cube groups
-    int* toff = nullptr;  // and the blocks' offsets
+    long long* toff = nullptr;  // and the blocks' offsets (five triangles a cube may pass 2^31)
     unsigned char* cases = nullptr;  // case byte per cube
     long long casecap = 0;
     float* tris = nullptr;
@@ -1184,15 +1184,16 @@ long long sphgpu_surface_mesh(sphgpu_surface_t s, float iso, int ref_rows, float
     ++s->kernels;
     k_mc_count<<<(int)nblocks, MCB, 0, st>>>(M, s->field, ngroups, gpr, s->cases, s->ntri);
     size_t b = 0;
-    cub::DeviceScan::ExclusiveSum(nullptr, b, s->ntri, s->toff, (int)nblocks, st);
+    const ::cuda::std::plus<> plus;
+    cub::DeviceScan::ExclusiveScan(nullptr, b, s->ntri, s->toff, plus, 0ll, (int)nblocks, st);
     if (int r = ensure_tmp(s, b)) return r;
-    cub::DeviceScan::ExclusiveSum(s->tmpbuf, b, s->ntri, s->toff, (int)nblocks, st);
-    int last_off = 0;
+    cub::DeviceScan::ExclusiveScan(s->tmpbuf, b, s->ntri, s->toff, plus, 0ll, (int)nblocks, st);
+    long long last_off = 0;
     int last_n = 0;
-    SCK(cudaMemcpyAsync(&last_off, s->toff + nblocks - 1, sizeof(int), cudaMemcpyDeviceToHost, st));
+    SCK(cudaMemcpyAsync(&last_off, s->toff + nblocks - 1, sizeof(long long), cudaMemcpyDeviceToHost, st));
     SCK(cudaMemcpyAsync(&last_n, s->ntri + nblocks - 1, sizeof(int), cudaMemcpyDeviceToHost, st));
     SCK(cudaStreamSynchronize(st));
-    const long long total = (long long)last_off + last_n;  // < 2^31: 5 triangles per cube at most
+    const long long total = last_off + last_n;
     s->ntris = total;
     if (total == 0) return 0;
     if (total > s->tricap) {

@@ -76,3 +76,27 @@ def test_mesh_after_no_memory_for_triangles():
     sf.set_field(few)
     np.testing.assert_array_equal(sf.mesh(0.5), want)
     sf.close()
+
+
+def test_more_than_2_31_triangles():
+    """A checkerboard of 814^3 nodes: four lone corners, so four triangles, in
+    every cube (77 GB of them on the device)."""
+    import ctypes as C
+    import torch
+    from graphics_b200.surface import surface_field
+    if torch.cuda.mem_get_info()[0] < 100e9:
+        pytest.skip("needs 100 GB of device memory")
+    heads = []
+    for n in (34, 814):
+        sf = surface_field()
+        sf.surface_setup([0.0] * 3, [0.01 * (n - 1) - 0.025] * 3, 0.01, 0.02, 0.01)
+        assert [int(v) for v in sf.grid_num] == [n] * 3
+        i = np.arange(n)
+        f = ((i[:, None, None] + i[None, :, None] + i[None, None, :]) & 1).astype(np.float32)
+        sf.set_field(f)
+        head = np.zeros((8, 3, 3), np.float32)
+        total = sf.lib.sphgpu_surface_mesh(sf.h, 0.5, 0, head.ctypes.data_as(C.POINTER(C.c_float)), len(head))
+        sf.close()
+        assert total == 4 * (n - 1) ** 3
+        heads.append(head)
+    np.testing.assert_array_equal(*heads)
