@@ -464,13 +464,13 @@ __global__ void k_sf_tile_count(const int4* box_lo, const int4* box_hi, int n, i
     npair[i] = tile_span(lo, hi, 0) * tile_span(lo, hi, 1) * tile_span(lo, hi, 2);
 }
 
-__global__ void k_sf_tile_emit(SfParams P, const int4* box_lo, const int4* box_hi, int n, const int* off, int* ptile,
-                               int* ppart) {
+__global__ void k_sf_tile_emit(SfParams P, const int4* box_lo, const int4* box_hi, int n, const long long* off,
+                               int* ptile, int* ppart) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int4 lo = box_lo[i], hi = box_hi[i];
     if (hi.x < lo.x || hi.y < lo.y || hi.z < lo.z) return;
-    int o = off[i];
+    int o = (int)off[i];
     for (int tz = lo.z / TZ; tz <= hi.z / TZ; ++tz)
         for (int ty = lo.y / TY; ty <= hi.y / TY; ++ty)
             for (int tx = lo.x / TX; tx <= hi.x / TX; ++tx) {
@@ -810,7 +810,8 @@ struct sphgpu_surface {
     double* mom = nullptr;  // 6 per particle
     float4 *pos = nullptr, *rec0 = nullptr, *rec1 = nullptr, *rec2 = nullptr;
     int4 *blo = nullptr, *bhi = nullptr;
-    int *key = nullptr, *slot = nullptr, *tmp = nullptr, *npair = nullptr, *poff = nullptr;
+    int *key = nullptr, *slot = nullptr, *tmp = nullptr, *npair = nullptr;
+    long long* poff = nullptr;  // the particles' first pairs, and their number
     int* pcnt = nullptr;    // neighbour-grid cells + 2
     int* pstart = nullptr;
     int* bad = nullptr;
@@ -931,13 +932,16 @@ int run_field(sphgpu_surface* s, int n, int aniso) {
         k_sf_tile_count<<<nblk(n, 256), 256, 0, st>>>(s->blo, s->bhi, n, s->npair);
         SCK(cudaMemsetAsync(s->npair + n, 0, sizeof(int), st));
         size_t b = 0;
-        cub::DeviceScan::ExclusiveSum(nullptr, b, s->npair, s->poff, n + 1, st);
+        const ::cuda::std::plus<> plus;
+        cub::DeviceScan::ExclusiveScan(nullptr, b, s->npair, s->poff, plus, 0ll, n + 1, st);
         if (int r = ensure_tmp(s, b)) return r;
-        cub::DeviceScan::ExclusiveSum(s->tmpbuf, b, s->npair, s->poff, n + 1, st);
-        int tot = 0;
-        SCK(cudaMemcpyAsync(&tot, s->poff + n, sizeof(int), cudaMemcpyDeviceToHost, st));
+        cub::DeviceScan::ExclusiveScan(s->tmpbuf, b, s->npair, s->poff, plus, 0ll, n + 1, st);
+        SCK(cudaMemcpyAsync(&npairs, s->poff + n, sizeof(long long), cudaMemcpyDeviceToHost, st));
         SCK(cudaStreamSynchronize(st));
-        npairs = tot;
+        if (npairs > 0x7fffffffll) {
+            s->err = "more than 2^31 - 1 (tile, particle) pairs";
+            return SPHGPU_EINVAL;
+        }
     }
     if (npairs > s->paircap) {
         const long long cap = std::max(npairs, 2 * s->paircap);

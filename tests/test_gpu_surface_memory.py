@@ -100,3 +100,22 @@ def test_more_than_2_31_triangles():
         assert total == 4 * (n - 1) ** 3
         heads.append(head)
     np.testing.assert_array_equal(*heads)
+
+
+def test_more_than_2_31_tile_pairs_are_refused():
+    """300 000 particles at one place, each over more than 8000 tiles; the
+    handle then makes another field."""
+    from graphics_b200.surface import surface_field
+    sf = surface_field()
+    sf.surface_setup([0.0] * 3, [0.02] * 3, 0.01, 0.02, 0.02 / 128)
+    one = np.full((1, 3), 0.01, np.float32)
+    assert sf.surface_isotro(one) == 0
+    want, pairs = sf.get_field(), sf.stats()[0]
+    n = 300_000
+    assert n * pairs > 2 ** 31
+    with pytest.raises(SphGpuError) as e:
+        sf.surface_isotro(np.repeat(one, n, 0))
+    assert e.value.code == _lib.EINVAL
+    assert sf.surface_isotro(one) == 0
+    np.testing.assert_array_equal(sf.get_field(), want)
+    sf.close()
