@@ -201,6 +201,14 @@ __global__ void k_sf_rank(const int* key, const int* start, const int* tmp, cons
     spos[a + r] = make_float4(p.x, p.y, p.z, __int_as_float(i));
 }
 
+// The covariance waits in the memory of records that only the decomposition
+// writes (rec2 and the node box, 16 bytes each): a buffer of its own was 48 bytes
+// a particle more to allocate in a handle's first field.
+struct Mom {
+    double2* v[3];
+    __device__ __forceinline__ double& at(int i, int l) const { return reinterpret_cast<double*>(v[l >> 1] + i)[l & 1]; }
+};
+
 // Moments of the anisotropic kernels, eight threads per particle: the
 // neighbours within h_field are collected in shared memory with their weights
 // 1 - (r/h_field)^3 (Equation 11), eight candidates at a time in cell order,
@@ -208,12 +216,12 @@ __global__ void k_sf_rank(const int* key, const int* start, const int* tmp, cons
 // covariance about their mean (FP64), each its own sum in that order.  The
 // 3 cells along x of a row of cells are one range of the cell order.  Out:
 // rec0 = (mean offset, sum of weights), the neighbour count, and with at least
-// n_e neighbours the unnormalised covariance xx, xy, xz, yy, yz, zz.
+// n_e neighbours the unnormalised covariance xx, xy, xz, yy, yz, zz (Mom).
 // 46 656 particles: 46 us, and 11 us for the decomposition after it (240 us with
 // both in one thread per particle, over all candidates twice).
 constexpr int ML = 8, MNT = 128, MCAP = 64;
 __global__ void __launch_bounds__(MNT) k_sf_moments(SfParams P, const float4* spos, int n, const int* start,
-                                                    float4* rec0, int* count, double* mom) {
+                                                    float4* rec0, int* count, Mom mom) {
     __shared__ float4 list[MNT / ML][MCAP];
     __shared__ int2 range[MNT / ML][9];  // {cell-order index - position in the candidates, positions up to its end}
     const int l = threadIdx.x % ML, grp = threadIdx.x / ML, q = blockIdx.x * (MNT / ML) + grp;
@@ -310,7 +318,7 @@ __global__ void __launch_bounds__(MNT) k_sf_moments(SfParams P, const float4* sp
             scan(cov);
         }
         cov();
-        if (l < 6 && wide) mom[6 * (size_t)__float_as_int(pi.w) + l] = C;
+        if (l < 6 && wide) mom.at(__float_as_int(pi.w), l) = C;
     }
     if (q < n && l == 6) {
         rec0[__float_as_int(pi.w)] = make_float4(mx, my, mz, sw);
@@ -357,10 +365,10 @@ __device__ void jacobi3(double m[3][3], double v[3][3]) {
 
 // Per particle: centre, G (symmetric, 6 values), det G, node box.
 // rec0 = (cx, cy, cz, det), rec1 = (gxx, gxy, gxz, gyy), rec2 = (gyz, gzz, -, -),
-// box_lo / box_hi = inclusive node ranges; rec0, count and mom hold the
-// particle's moments before.
+// box_lo / box_hi = inclusive node ranges; rec0, count and mom (in rec2,
+// box_lo and box_hi) hold the particle's moments before.
 __global__ void __launch_bounds__(64) k_sf_kernel(SfParams P, const float4* pos, int n, int aniso, const int* count,
-                                                  const double* mom, float4* rec0, float4* rec1, float4* rec2,
+                                                  Mom mom, float4* rec0, float4* rec1, float4* rec2,
                                                   int4* box_lo, int4* box_hi) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -375,8 +383,8 @@ __global__ void __launch_bounds__(64) k_sf_kernel(SfParams P, const float4* pos,
         if (nn >= P.n_e) {
             const float4 mean = rec0[i];
             const float mx = mean.x, my = mean.y, mz = mean.z, sw = mean.w;
-            const double* c = mom + 6 * (size_t)i;
-            double C[3][3] = {{c[0], c[1], c[2]}, {0, c[3], c[4]}, {0, 0, c[5]}};
+            const double2 c0 = mom.v[0][i], c1 = mom.v[1][i], c2 = mom.v[2][i];
+            double C[3][3] = {{c0.x, c0.y, c1.x}, {0, c1.y, c2.x}, {0, 0, c2.y}};
             C[1][0] = C[0][1];
             C[2][0] = C[0][2];
             C[2][1] = C[1][2];
@@ -807,7 +815,6 @@ struct sphgpu_surface {
     // particles
     int pcap = 0;
     float* xyz = nullptr;  // host positions staged on the device
-    double* mom = nullptr;  // 6 per particle
     float4 *pos = nullptr, *rec0 = nullptr, *rec1 = nullptr, *rec2 = nullptr;
     int4 *blo = nullptr, *bhi = nullptr;
     int *key = nullptr, *slot = nullptr, *tmp = nullptr, *npair = nullptr;
@@ -889,7 +896,7 @@ int ensure_particles(sphgpu_surface* s, int n) {
     s->pcap = 0;
     int r = salloc(s, &s->pos, cap) | salloc(s, &s->rec0, cap) | salloc(s, &s->rec1, cap) | salloc(s, &s->rec2, cap) |
             salloc(s, &s->blo, cap) | salloc(s, &s->bhi, cap) | salloc(s, &s->key, cap) | salloc(s, &s->slot, cap) |
-            salloc(s, &s->tmp, cap) | salloc(s, &s->mom, 6 * (size_t)cap) | salloc(s, &s->npair, (size_t)cap + 1) |
+            salloc(s, &s->tmp, cap) | salloc(s, &s->npair, (size_t)cap + 1) |
             salloc(s, &s->poff, (size_t)cap + 1) | salloc(s, &s->xyz, 3 * (size_t)cap);
     if (r) return SPHGPU_ENOMEM;
     s->pcap = cap;
@@ -906,6 +913,7 @@ int run_field(sphgpu_surface* s, int n, int aniso) {
     cudaStream_t st = s->stream;
     const SfParams& P = s->P;
     const int pcells = P.pnum[0] * P.pnum[1] * P.pnum[2];
+    const Mom mom{{(double2*)s->rec2, (double2*)s->blo, (double2*)s->bhi}};
     // neighbour grid (anisotropic kernels only)
     if (aniso && n > 0) {
         float4* const spos = s->rec1;  // positions in cell order until k_sf_kernel writes the record
@@ -919,11 +927,11 @@ int run_field(sphgpu_surface* s, int n, int aniso) {
         cub::DeviceScan::ExclusiveSum(s->tmpbuf, b, s->pcnt, s->pstart, pcells + 2, st);
         k_sf_scatter<<<nblk(n, 256), 256, 0, st>>>(s->key, s->slot, s->pstart, n, s->tmp);
         k_sf_rank<<<nblk(n, 256), 256, 0, st>>>(s->key, s->pstart, s->tmp, s->pos, n, spos);
-        k_sf_moments<<<nblk(n, MNT / ML), MNT, 0, st>>>(P, spos, n, s->pstart, s->rec0, s->npair, s->mom);
+        k_sf_moments<<<nblk(n, MNT / ML), MNT, 0, st>>>(P, spos, n, s->pstart, s->rec0, s->npair, mom);
     }
     s->kernels += n > 0;
     if (n > 0)
-        k_sf_kernel<<<nblk(n, 64), 64, 0, st>>>(P, s->pos, n, aniso, s->npair, s->mom, s->rec0, s->rec1, s->rec2,
+        k_sf_kernel<<<nblk(n, 64), 64, 0, st>>>(P, s->pos, n, aniso, s->npair, mom, s->rec0, s->rec1, s->rec2,
                                                 s->blo, s->bhi);
     // tile pairs
     long long npairs = 0;
@@ -1060,7 +1068,7 @@ int sphgpu_surface_create(const double* mn, const double* mx, double r_p, double
 int sphgpu_surface_destroy(sphgpu_surface_t s) {
     if (!s) return SPHGPU_EINVAL;
     cudaSetDevice(s->device);
-    void* ptrs[] = {s->field, s->xyz, s->pos, s->rec0, s->rec1, s->rec2, s->blo, s->bhi, s->key, s->slot, s->tmp, s->mom,
+    void* ptrs[] = {s->field, s->xyz, s->pos, s->rec0, s->rec1, s->rec2, s->blo, s->bhi, s->key, s->slot, s->tmp,
                     s->npair, s->poff, s->pcnt, s->pstart, s->bad, s->ptile, s->ppart, s->ptile_s, s->ppart_s,
                     s->tstart, s->ntri, s->toff, s->cases, s->tris, s->coords, s->tmpbuf};
     for (void* p : ptrs)
