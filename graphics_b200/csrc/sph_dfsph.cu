@@ -27,20 +27,6 @@
 namespace {
 constexpr int NT = 128;
 
-__global__ void k_step_begin(DevScene s) { stats_step_begin(s.st); }
-
-// per-call counters: status bits are OR-ed and removals / dropped pairs
-// summed over all steps of one API call
-__global__ void k_call_begin(DevScene s) {
-    DevStats* st = s.st;
-    st->removed = 0;
-    st->overflow = 0;
-    st->zero_dis = 0;
-    st->status = 0u;
-    st->total_it_density = 0;
-    st->total_it_div = 0;
-}
-
 // non-pressure accelerations (gravity + viscosity) and v_adv.  The list is
 // read four entries at a time (one 16-byte load, the next group's issued
 // before the current group's record gathers) and each neighbour costs one
@@ -679,9 +665,6 @@ static inline int nblk(int n, int bs = NT) { return (n > 0 ? n + bs - 1 : bs) / 
         case 256: { constexpr int B = 256; CALL; break; } \
         default: { constexpr int B = 128; CALL; break; }  \
     }
-
-void launch_step_begin(const DevScene& s, cudaStream_t st) { k_step_begin<<<1, 1, 0, st>>>(s); }
-void launch_call_begin(const DevScene& s, cudaStream_t st) { k_call_begin<<<1, 1, 0, st>>>(s); }
 
 // the kernels with four threads per particle: 64 or 128 threads (their rows of
 // factors fit the default shared memory)

@@ -1389,7 +1389,6 @@ static int create_impl(const SphParams* p, int device, int max_fluid, int nscene
     fill_solver_const(h);
     mlp_init_attributes();
     ws_init_attributes();
-    warp_build_init();
     int r = alloc_scene(h);
     if (!r && nscenes > 1) {
         // per-scene state: grids, then one block for the BatchDev arrays

@@ -264,6 +264,8 @@ __device__ __forceinline__ void walk4(const int* list, size_t stride, int p, int
 }
 
 // ---- neighbour search (sph_grid.cu) ----
+void launch_step_begin(const DevScene& s, cudaStream_t st);
+void launch_call_begin(const DevScene& s, cudaStream_t st);
 // integrate: bit 0 the DFSPH position update, bit 1 carry cA, bit 2 the
 // learned warm start's history from this step's sums (k_ws_post's job), bit 3
 // the step begins here (stats_step_begin)
@@ -276,11 +278,10 @@ void launch_scatter_reorder(const DevScene& s, const GridGeom& g, int n_old, int
 // 22.7 us at 1.7 k keys, 32.0 / 31.2 at 4 k, 47.4 / 47.3 at 8 k, 84 / 90 at 14 k)
 constexpr int SCAN_MAX = 1 << 13;
 void launch_scan(const DevScene& s, const GridGeom& g, cudaStream_t st);
-// ---- list build, a warp per particle (sph_warp.cu) ----
-void launch_warp_build(const DevScene& s, const GridGeom& g, const SolverConst& c, int mode, int n_max, cudaStream_t st,
-                       int bs);
-int warp_build_blocks(int n_max, int bs);
-void warp_build_init();
+// ---- list build, a warp for a few particles (sph_warp.cu) ----
+void launch_warp_build(const DevScene& s, const GridGeom& g, const SolverConst& c, int mode, int n_max,
+                       cudaStream_t st);
+int warp_build_blocks(int n_max);
 void launch_build(const DevScene& s, const GridGeom& g, const SolverConst& c, int mode, int n_max, cudaStream_t st,
                   int bs = 128);
 void launch_to_ref_order(const float4* src, const int* gid, int n, float* dst3, cudaStream_t st);
@@ -320,8 +321,6 @@ void launch_df_div_b(const DevScene& s, const SolverConst& c, int n_max, int par
                      int bs = 128);
 void launch_df_warm_correction(const DevScene& s, const SolverConst& c, int n_max, cudaStream_t st, int bs = 128);
 void launch_cfl(const DevScene& s, int n_max, float cfl, float d, float dt_max, float dt_min, cudaStream_t st);
-void launch_step_begin(const DevScene& s, cudaStream_t st);
-void launch_call_begin(const DevScene& s, cudaStream_t st);
 
 // ---- batch of scenes (sph_batch.cu) ----
 void launch_batch_loop_reset(const DevScene& s, int nscenes, int which, cudaStream_t st);

@@ -36,10 +36,17 @@ struct WarpSmem {
     float sum[GROUP * SUMS];
 };
 
-template <int MODE, int BS>
-__global__ void __launch_bounds__(BS) k_warp_build(const __grid_constant__ DevScene s, const __grid_constant__ GridGeom g,
+// One block size: its warps share nothing but the statistics, and 64 or 256
+// threads are no faster (event-timed 64 / 128 / 256: 1 k particles 12.7 / 12.7 /
+// 12.7 us, 8 k 19.1 / 18.9 / 20.8, 27 k 36 / 36 / 40, 46 k 49 / 49 / 53, 64 k
+// 78 / 78 / 83), while every instantiation makes the module longer that a
+// process loads for its first small scene.
+constexpr int NT = 128;
+
+template <int MODE>
+__global__ void __launch_bounds__(NT) k_warp_build(const __grid_constant__ DevScene s, const __grid_constant__ GridGeom g,
                                                    const __grid_constant__ SolverConst c, int group) {
-    constexpr int WPB = BS / 32;
+    constexpr int WPB = NT / 32;
     using Smem = WarpSmem<MODE>;
     extern __shared__ int4 warp_smem[];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -222,9 +229,9 @@ __global__ void __launch_bounds__(BS) k_warp_build(const __grid_constant__ DevSc
         }
     }
     __shared__ int sh[WPB];
-    const int tot = block_sum_int<BS>(ntot, sh);
-    const int ov = block_sum_int<BS>(over, sh);
-    const int mx = block_max_int<BS>(nmax, sh);
+    const int tot = block_sum_int<NT>(ntot, sh);
+    const int ov = block_sum_int<NT>(over, sh);
+    const int mx = block_max_int<NT>(nmax, sh);
     if (threadIdx.x == 0) {
         if (tot) atomicAdd(&s.st->nbr_total, (unsigned long long)tot);
         if (ov) { atomicAdd(&s.st->overflow, ov); atomicOr(&s.st->status, 8u); }
@@ -234,44 +241,23 @@ __global__ void __launch_bounds__(BS) k_warp_build(const __grid_constant__ DevSc
         // the block's part of the iteration's FP64 sum of Drho/Dt (as
         // k_df_div_a; a batch, mode 5, reduces per scene in batch_decide)
         __shared__ double shd[WPB];
-        const double bsum = block_sum_double<BS>(dsum, shd);
+        const double bsum = block_sum_double<NT>(dsum, shd);
         if (threadIdx.x == 0) s.partial[blockIdx.x] = bsum;
     }
 }
 }  // namespace
 
-#define EACH_MODE(DO) DO(0) DO(1) DO(2) DO(3) DO(4) DO(5)
-
 // particles per warp: enough warps for every SM first
 static int warp_group(int n_max) { return std::min(GROUP, std::max(1, n_max / (148 * 16))); }
-int warp_build_blocks(int n_max, int bs) {
-    const int per = (bs == 64 || bs == 256 ? bs : 128) / 32 * warp_group(n_max), n = n_max > 0 ? n_max : 1;
+int warp_build_blocks(int n_max) {
+    const int per = NT / 32 * warp_group(n_max), n = n_max > 0 ? n_max : 1;
     return (n + per - 1) / per;
 }
 
-void launch_warp_build(const DevScene& s, const GridGeom& g, const SolverConst& c, int mode, int n_max, cudaStream_t st,
-                       int bs) {
+void launch_warp_build(const DevScene& s, const GridGeom& g, const SolverConst& c, int mode, int n_max, cudaStream_t st) {
     if (mode == 4 && s.nscenes > 1) mode = 5;
-    const int group = warp_group(n_max), nb = warp_build_blocks(n_max, bs);
-#define GO(M, B) k_warp_build<M, B><<<nb, B, sizeof(WarpSmem<M>) * (B / 32), st>>>(s, g, c, group)
-#define ONE(M)                          \
-    case M:                             \
-        if (bs == 64) GO(M, 64);        \
-        else if (bs == 256) GO(M, 256); \
-        else GO(M, 128);                \
-        break;
-    switch (mode) { EACH_MODE(ONE) }
-#undef ONE
-#undef GO
-}
-
-// more shared memory than the default limit at 256 threads; also loads every
-// instantiation (see preload_sweep_kernels)
-void warp_build_init() {
-#define ONE(M, B) \
-    cudaFuncSetAttribute(k_warp_build<M, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(WarpSmem<M>) * (B / 32));
-#define ALL(M) ONE(M, 64) ONE(M, 128) ONE(M, 256)
-    EACH_MODE(ALL)
-#undef ALL
+    const int group = warp_group(n_max), nb = warp_build_blocks(n_max);
+#define ONE(M) case M: k_warp_build<M><<<nb, NT, sizeof(WarpSmem<M>) * (NT / 32), st>>>(s, g, c, group); break;
+    switch (mode) { ONE(0) ONE(1) ONE(2) ONE(3) ONE(4) ONE(5) }
 #undef ONE
 }
