@@ -28,13 +28,15 @@ template <int MODE>
 struct WarpSmem {
     static constexpr int N = MODE ? BuildSums<MODE ? MODE : 1>::N : 1;
     static constexpr int PAIR = MODE ? 2 : 0;  // particles whose sums run together
-    int list[GROUP * LIST];
+    alignas(16) int list[GROUP * LIST];        // read as int4
     union {
         int cand[WINDOW];
         float uv[(PAIR ? PAIR : 1) * 2 * N * TROW];
     };
     float sum[GROUP * SUMS];
 };
+static_assert(LIST % 4 == 0 && sizeof(WarpSmem<0>) % 16 == 0 && sizeof(WarpSmem<3>) % 16 == 0,
+              "every particle's row of every warp's list on 16 bytes");
 
 // One block size: its warps share nothing but the statistics, and 64 or 256
 // threads are no faster (event-timed 64 / 128 / 256: 1 k particles 12.7 / 12.7 /
