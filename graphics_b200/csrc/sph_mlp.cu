@@ -24,7 +24,7 @@
 
 namespace {
 
-constexpr int TR = 128;  // rows per block tile (4 warps x 32)
+constexpr int TR = 128;  // rows per block tile
 
 // GELU in its tanh form, 0.5 z (1 + tanh(sqrt(2/pi) (z + 0.044715 z^3))),
 // with the hardware tanh (PTX tanh.approx.f32, relative error about 2^-11,
@@ -113,7 +113,6 @@ struct FwdSmem {
     __nv_bfloat16 W1[MLP_IN * MLP_H];
     __nv_bfloat16 W2[MLP_H * MLP_H];
     __nv_bfloat16 H1[TR * MLP_H];
-    float Z1[TR * MLP_H];
     float Z2[TR * MLP_H];
     float W3[MLP_H], b1[MLP_H], b2[MLP_H];
     float b3;
@@ -131,22 +130,18 @@ __device__ __forceinline__ void load_weights(const MlpDev& m, FwdSmem& S) {
     if (threadIdx.x == 0) S.b3 = m.master[MLP_OFF_B3];
 }
 
-// Forward pass of the warp's 32 rows (S.X filled, weights loaded):
-// Z1, H1 (BF16), Z2 in shared memory; returns y for row lane of the warp.
+// Prediction's forward pass of the warp's 32 rows (S.X filled, weights loaded):
+// H1 (BF16) and Z2 in shared memory; returns y for row lane of the warp.
 __device__ __forceinline__ float forward_rows(FwdSmem& S) {
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const int r0 = w * 32;
-    // layer 1: Z1 = X W1 + b1   (K = 16)
+    // layer 1: H1 = GELU(X W1 + b1)   (K = 16)
     for (int mt = 0; mt < 2; ++mt)
         for (int nt = 0; nt < MLP_H / 8; ++nt) {
             float c[4] = {0.f, 0.f, 0.f, 0.f};
             tile_mma(c, S.X, MLP_IN, 1, S.W1, MLP_H, 1, r0 + mt * 16, nt * 8, MLP_IN);
             const int ra = r0 + mt * 16 + g, col = nt * 8 + 2 * t;
             const float z[4] = {c[0] + S.b1[col], c[1] + S.b1[col + 1], c[2] + S.b1[col], c[3] + S.b1[col + 1]};
-            S.Z1[ra * MLP_H + col] = z[0];
-            S.Z1[ra * MLP_H + col + 1] = z[1];
-            S.Z1[(ra + 8) * MLP_H + col] = z[2];
-            S.Z1[(ra + 8) * MLP_H + col + 1] = z[3];
             S.H1[ra * MLP_H + col] = __float2bfloat16_rn(gelu(z[0]));
             S.H1[ra * MLP_H + col + 1] = __float2bfloat16_rn(gelu(z[1]));
             S.H1[(ra + 8) * MLP_H + col] = __float2bfloat16_rn(gelu(z[2]));
