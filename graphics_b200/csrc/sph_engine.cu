@@ -264,10 +264,17 @@ GridGeom make_grid(const SphParams& P) {
 // lanes wait for: 1 k 44 / 10, 64 k 54 / 37, 97 k 57 / 45, 125 k 59 / 61, 166 k
 // 78 / 65, 262 k 99 / 98, 405 k 139 / 149
 constexpr int WARP_BUILD_MAX = 65536, WARP_LISTS_MAX = 262144;
-// WCSPH's force pass runs four threads per particle up to this capacity
-// (event-timed, one / four: 27 k 14.7 / 10.9 us, 47 k 15.9 / 14.6, 64 k 16.7 /
-// 16.7, 80 k 18.8 / 20.8, 262 k 40 / 46)
-constexpr int WC_LANES_MAX = 65536;
+// WCSPH with surface tension or adhesion
+bool wc_surface(const SphParams& P) { return P.th_h != 0.f || P.th_r != 0.f || P.th_bt != 0.f; }
+// WCSPH's force pass runs four threads per particle up to these capacities: the
+// plain one, a record per neighbour and four in flight (event-timed, one / four:
+// 27 k 14.7 / 10.9 us, 47 k 15.9 / 14.6, 64 k 16.7 / 16.7, 80 k 18.8 / 20.8, 262 k
+// 40 / 46), and the general one of several fluids or surface terms, whose thread
+// waits out each neighbour's gathers in turn (whole step, two fluids: 80 k 133 /
+// 111 us, 141 k 153 / 146, 227 k 228 / 212, 262 k 240 / 230; surface terms 80 k
+// 168 / 146, 141 k 186 / 180, 262 k 300 / 293).
+// By capacity, like the rules above, not by count: a snapshot resumes the same.
+constexpr int WC_LANES_MAX = 65536, WC_GENERAL_LANES_MAX = 262144;
 // Capacities up to which the DFSPH sweeps run four threads per particle
 // (forces and the A sweeps; the B sweeps); both sides measured in sph_dfsph.cu
 constexpr int LANES_A_MAX = 24000, LANES_B_MAX = 12000;
@@ -312,7 +319,8 @@ void fill_solver_const(sphgpu_scene* h) {
                               : (h->cap <= WARP_BUILD_MAX ? 1 : (h->cap <= WARP_LISTS_MAX ? 2 : 0));
     c.stride = h->stride;
     c.l2pol = h->l2pol;
-    c.lanes = h->wc_lanes ? h->wc_lanes : (h->cap <= WC_LANES_MAX ? 4 : 1);
+    const bool wc_general = c.nphase > 1 || wc_surface(P);
+    c.lanes = h->wc_lanes ? h->wc_lanes : (h->cap <= (wc_general ? WC_GENERAL_LANES_MAX : WC_LANES_MAX) ? 4 : 1);
     const bool lanes_ok = h->ncap <= 48;  // a particle's factors fit its shared-memory row
     c.lanes_a = lanes_ok && (h->sweep_lanes ? h->sweep_lanes == 4 : h->cap <= LANES_A_MAX) ? 4 : 1;
     c.lanes_b = lanes_ok && (h->sweep_lanes ? h->sweep_lanes == 4 : h->cap <= LANES_B_MAX) ? 4 : 1;
@@ -869,7 +877,7 @@ int enq_iv_step(sphgpu_scene* h, bool capturing) {
 int enq_wc_step(sphgpu_scene* h, bool, bool copy_stats = true) {
     cudaStream_t st = h->stream;
     enq_ns(h, 8, 2, st);
-    const bool surf = h->P.th_h != 0.f || h->P.th_r != 0.f || h->P.th_bt != 0.f;
+    const bool surf = wc_surface(h->P);
     if (surf) launch(h, "wc_normal", st, [&] { launch_wc_normal(h->d, h->c, h->cap, st); });
     launch(h, "wc_force", st, [&] { launch_wc_force(h->d, h->c, h->cap, st, surf, h->c.lanes); });
     if (copy_stats) CK(cudaMemcpyAsync(h->h_stats, h->d.st, sizeof(DevStats), cudaMemcpyDeviceToHost, st));
@@ -2275,7 +2283,7 @@ int sphgpu_stage(sphgpu_t h, const char* name, SphStepStats* stats) {
         h->ep_acc = h->ep_loop = h->sorts;
     } else if (s == "wc_computeForce") {
         if (h->in_staging) { h->err = "run neighbourSearch first"; return SPHGPU_EINVAL; }
-        const bool surf = h->P.th_h != 0.f || h->P.th_r != 0.f || h->P.th_bt != 0.f;
+        const bool surf = wc_surface(h->P);
         if (surf) launch_wc_normal(d, h->c, h->cap, st);
         launch_wc_records(d, h->cap, st);
         launch_wc_force(d, h->c, h->cap, st, surf, h->c.lanes);

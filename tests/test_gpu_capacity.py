@@ -67,6 +67,31 @@ def test_lists_alone_by_warps(solver):
     _same(_run(solver, knobs=[("build", 0)]), _run(solver, knobs=[("build", 2)]))
 
 
+# threads per particle of WCSPH's force pass (they differ in the order of the
+# sums): the plain pass, two fluids, surface terms, on both sides of their lines
+@pytest.mark.parametrize("kind,cap,lanes", [("plain", 65_536, 4), ("plain", 65_537, 1), ("two", 65_537, 4),
+                                            ("two", 262_144, 4), ("two", 262_145, 1), ("surface", 65_537, 4),
+                                            ("surface", 262_145, 1)])
+def test_threads_per_particle_of_the_wcsph_forces(kind, cap, lanes):
+    sc = _scene("pcisph" if kind == "two" else "dfsph")
+    kw = dict(dt=2.5e-4, soundSpeed_cs=18.0)
+    if kind == "surface":
+        kw.update(th_h=sc.smooth_radius, th_r=0.2, th_bt=1.0)
+    out = []
+    for forced in (0, lanes, 5 - lanes):
+        g = GpuScene(params_for_scene(sc, **kw), cap)
+        g.debug_set("wc_lanes", forced)
+        g.set_boundary(sc.boundary_pos)
+        phase = np.zeros(sc.n_fluid, np.int32) if sc.phase is None else sc.phase
+        for ph, rho in enumerate(sc.rho0_phases):
+            g.add_fluid(sc.fluid_pos[phase == ph], sc.fluid_vel[phase == ph], rho0=rho, visc_alpha=0.05)
+        g.step("wcsph", 1)
+        out.append(g.get("acceleration"))
+        g.close()
+    np.testing.assert_array_equal(out[0], out[1])
+    assert not np.array_equal(out[0], out[2])
+
+
 def test_unknown_list_builds_are_refused():
     sc = _scene("dfsph", (2, 2, 2))
     g = GpuScene(params_for_scene(sc, **DF), sc.n_fluid)
