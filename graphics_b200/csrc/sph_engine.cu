@@ -260,7 +260,8 @@ GridGeom make_grid(const SphParams& P) {
 // thread / warp, event-timed: DFSPH rho + alpha + first divergence sweep 1 k
 // particles 52 / 14 us, 8 k 54 / 25, 27 k 57 / 41, 64 k 66 / 66, 125 k
 // 85 / 114; WCSPH 27 k 48 / 28, 47 k 52 / 37, 64 k 55 / 57, 80 k 55 / 62,
-// 262 k 110 / 150.  Lists alone (PCISPH, IISPH_M) carry no sums that idle
+// 262 k 110 / 150; IISph 1 k 53 / 11, 27 k 57 / 32, 47 k 62 / 42, 64 k 65 / 65, 80 k
+// 67 / 70, 125 k 73 / 100, 262 k 127 / 171.  Lists alone (PCISPH, IISPH_M) carry no sums that idle
 // lanes wait for: 1 k 44 / 10, 64 k 54 / 37, 97 k 57 / 45, 125 k 59 / 61, 166 k
 // 78 / 65, 262 k 99 / 98, 405 k 139 / 149
 constexpr int WARP_BUILD_MAX = 65536, WARP_LISTS_MAX = 262144;

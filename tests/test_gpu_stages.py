@@ -35,3 +35,26 @@ def test_wcsph_forces_after_set_density(lanes):
         g.close()
     # some 50 terms, each a few ulp of the largest, in either pass: 50 * 4 * 2^-24
     assert np.abs(acc[0] - acc[1]).max() <= 50 * 4 * 2.0 ** -24 * np.abs(acc[0]).max()
+
+
+# the list build of the pressure stage, by a thread and by a warp for a few
+# particles: lists, densities and pressures, also over the cap (a block squeezed
+# to two thirds) and with a short one
+@pytest.mark.parametrize("squeeze,cap", [(1.0, 48), (0.66, 48), (1.0, 10)])
+def test_wcsph_pressure_stage_by_either_list_build(squeeze, cap):
+    r, counts = 0.0125, (12, 11, 13)
+    sc = dam_break(counts, r, tuple(2 * r * (k + 3) for k in counts), seed=5)
+    out = []
+    for build in (0, 1):
+        g = GpuScene(params_for_scene(sc, dt=2.5e-4, soundSpeed_cs=18.0, max_neighbours=cap), sc.n_fluid)
+        g.debug_set("build", build)
+        g.set_boundary(sc.boundary_pos)
+        g.add_fluid((sc.fluid_pos * np.float32(squeeze)).astype(np.float32), sc.fluid_vel)
+        g.stage("wc_computePressure")
+        count, kind, index = g.neighbours()
+        kept = np.arange(kind.shape[1])[None, :] < count[:, None]
+        assert count.max() == cap if squeeze < 1 or cap < 48 else count.max() < cap
+        out.append((count, kind[kept], index[kept], g.get("density"), g.get("presure")))
+        g.close()
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)
