@@ -475,8 +475,9 @@ __global__ void __launch_bounds__(TNT) k_mlp_train(MlpDev m, const float* X, con
 // Gradient of the mini-batch = the tiles' gradients summed in tile order, and
 // the batch's squared error, added to m.loss.  ADAM: the update of the FP32
 // master weights and the GEMMs' BF16 copies with it; else the gradient to
-// m.grad.  64 threads a block, 32 loads in flight each: 3.6 us alone
-// for one tile, against 4.3 + 1.8 us of a separate sum and Adam for 64 tiles.
+// m.grad.  64 threads a block, 32 loads in flight each: 6.5 us for 64 tiles
+// (one kernel at a time, caches cold), against 7.0 + 3.3 us of a separate sum
+// and Adam.
 constexpr int UNT = 64;
 template <bool ADAM>
 __global__ void __launch_bounds__(UNT) k_mlp_update(MlpDev m, int blocks, float lr, float bc1, float bc2) {

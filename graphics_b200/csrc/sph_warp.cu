@@ -2,7 +2,7 @@
 //
 // A thread per particle walks some 220 candidates and 30 neighbours one
 // after the other: a small scene has too few warps on the chip to hide that
-// (1 k particles: 47 us), and a large one spends its issue slots on the loop
+// (1 k particles: 44 to 53 us, by mode), and a large one spends its issue slots on the loop
 // and on the lanes that wait for the longest walk.  Here a warp takes up to
 // 16 consecutive sorted particles, cell by cell: the candidates of a cell
 // (its 27 cells' records, in the reference's order) go into the lanes'
