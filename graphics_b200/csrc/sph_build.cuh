@@ -17,8 +17,12 @@ constexpr bool build_has_div(int mode) { return mode == 4 || mode == 5; }
 
 // The sums a mode takes over a list, in list order, each a chain of
 // acc = fma(u, v, acc): 1: density, sum m gradW (3), sum |m gradW|^2 over
-// fluid; 2: density; 3: density, gamma, sphVolume, sum V gradW (3), sum
-// V^2 |gradW|^2 / m over fluid; 4 and 5: mode 1's and the divergence sum.
+// fluid; 2: density, in blocks of DENS_BLOCK entries whose sums are added in
+// turn, since the pressure is its seventh power (error against FP64, 30 blocks of
+// 1 000 particles: density 1.12e-7 rms so, 1.30e-7 in one chain; the pressures'
+// largest 4.3e-6 against 5.6e-6); 3: density, gamma, sphVolume, sum V gradW (3),
+// sum V^2 |gradW|^2 / m over fluid; 4 and 5: mode 1's and the divergence sum.
+constexpr int DENS_BLOCK = 8;
 template <int MODE>
 struct BuildSums {
     static constexpr int N = MODE == 2 ? 1 : MODE == 3 ? 7 : build_has_div(MODE) ? 6 : 5;
@@ -136,14 +140,33 @@ __device__ __forceinline__ void list_terms(const DevScene& s, const SolverConst&
     BuildSums<MODE> a;
     sums_begin<MODE>(c, pa, a);
     const float4 va = build_has_div(MODE) ? s.pv[2 * p + 1] : make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int k = 0; k < cnt; ++k) {
-        bool bnd;
-        float4 pb, vb;
-        fetch(k, bnd, pb, vb);
-        BuildSums<MODE> u, v;
-        pair_terms<MODE>(c, pa, va, bnd, pb, vb, u, v);
+    auto entries = [&](int k, int end, BuildSums<MODE>& t) {
+#pragma unroll 4
+        for (; k < end; ++k) {
+            bool bnd;
+            float4 pb, vb;
+            fetch(k, bnd, pb, vb);
+            BuildSums<MODE> u, v;
+            pair_terms<MODE>(c, pa, va, bnd, pb, vb, u, v);
 #pragma unroll
-        for (int i = 0; i < BuildSums<MODE>::N; ++i) a.v[i] = fmaf(u.v[i], v.v[i], a.v[i]);
+            for (int i = 0; i < BuildSums<MODE>::N; ++i) t.v[i] = fmaf(u.v[i], v.v[i], t.v[i]);
+        }
+    };
+    if (MODE == 2) {
+        // (whole blocks first: of a known length, so that their loads go together)
+        int k0 = 0;
+        for (; k0 + DENS_BLOCK <= cnt; k0 += DENS_BLOCK) {
+            BuildSums<MODE> t;
+            t.v[0] = 0.f;
+            entries(k0, k0 + DENS_BLOCK, t);
+            a.v[0] += t.v[0];
+        }
+        BuildSums<MODE> t;
+        t.v[0] = 0.f;
+        entries(k0, cnt, t);
+        a.v[0] += t.v[0];
+    } else {
+        entries(0, cnt, a);
     }
     ddiv = sums_finish<MODE>(s, c, p, pa, a);
 }

@@ -2,16 +2,16 @@
 //
 // A thread per particle walks some 220 candidates and 30 neighbours one
 // after the other: a small scene has too few warps on the chip to hide that
-// (1 k particles: 44 to 53 us, by mode), and a large one spends its issue slots on the loop
-// and on the lanes that wait for the longest walk.  Here a warp takes up to
-// 16 consecutive sorted particles, cell by cell: the candidates of a cell
-// (its 27 cells' records, in the reference's order) go into the lanes'
+// (1 k particles: 44 to 53 us, by mode), and a large one spends its issue slots
+// on the loop and on the lanes that wait for the longest walk.  Here a warp
+// takes up to 16 consecutive sorted particles, cell by cell: the candidates of a
+// cell (its 27 cells' records, in the reference's order) go into the lanes'
 // registers once, each particle of the cell tests 32 of them per
 // instruction, and a ballot gives every hit its place in the list.  Then the
 // lanes take one list entry each for the terms; the sums run in list order,
-// one lane per sum, so every result is the one k_build (sph_grid.cu) gives,
-// bit for bit: the same cells in the same order, the same float cut test,
-// the same cap.
+// one lane per sum (WCSPH's density: per block of it), so every result is the
+// one k_build (sph_grid.cu) gives, bit for bit: the same cells in the same
+// order, the same float cut test, the same cap.
 #include <algorithm>
 
 #include "sph_build.cuh"
@@ -161,14 +161,15 @@ __global__ void __launch_bounds__(NT) k_warp_build(const __grid_constant__ DevSc
         if (MODE != 0) {
             constexpr int M = MODE ? MODE : 1;
             constexpr int N = Smem::N, PAIR = MODE ? Smem::PAIR : 1;
+            constexpr int R = MODE == 2 ? (LIST - 4) / DENS_BLOCK : N;  // results per particle (cap <= LIST - 4)
             float4 va = make_float4(0.f, 0.f, 0.f, 0.f);
             if (build_has_div(MODE) && lane < ng) va = s.pv[2 * (p0 + lane) + 1];
             for (int j0 = 0; j0 < ng; j0 += PAIR) {
-                // lane b * SUMS + i: sum i of particle j0 + b
+                // lane b * SUMS + i: sum i (MODE 2: block i of the one sum) of particle j0 + b
                 const int b = lane / SUMS, i = lane % SUMS;
-                const bool sums = b < PAIR && i < N && j0 + b < ng;
+                const bool sums = b < PAIR && i < R && j0 + b < ng;
                 float acc = 0.f;
-                {
+                if (MODE != 2) {
                     BuildSums<M> a;
                     sums_begin<M>(c, make_float4(0.f, 0.f, 0.f, __shfl_sync(0xffffffffu, pa.w, (j0 + b) & 31)), a);
 #pragma unroll
@@ -210,10 +211,13 @@ __global__ void __launch_bounds__(NT) k_warp_build(const __grid_constant__ DevSc
                     }
                     __syncwarp();
                     if (sums) {
-                        const int end = min(32, mykept - k0);
-                        const float* const U = m.uv + 2 * (b * N + i) * TROW;
+                        // MODE 2: block i is DENS_BLOCK of these 32 entries or none
+                        const int first = MODE == 2 ? i * DENS_BLOCK - k0 : 0;
+                        const int end = min(MODE == 2 ? min(32, first + DENS_BLOCK) : 32, mykept - k0);
+                        const float* const U = m.uv + 2 * (b * N + (MODE == 2 ? 0 : i)) * TROW;
+                        if (first >= 0)
 #pragma unroll 4
-                        for (int k = 0; k < end; ++k) acc = fmaf(U[k], U[TROW + k], acc);
+                            for (int k = first; k < end; ++k) acc = fmaf(U[k], U[TROW + k], acc);
                     }
                     __syncwarp();
                 }
@@ -222,8 +226,12 @@ __global__ void __launch_bounds__(NT) k_warp_build(const __grid_constant__ DevSc
             __syncwarp();
             if (lane < ng) {
                 BuildSums<M> a;
+                if (MODE == 2) sums_begin<M>(c, pa, a);
 #pragma unroll
-                for (int q = 0; q < N; ++q) a.v[q] = m.sum[lane * SUMS + q];
+                for (int q = 0; q < R; ++q) {
+                    if (MODE == 2) a.v[0] += m.sum[lane * SUMS + q];
+                    else a.v[q] = m.sum[lane * SUMS + q];
+                }
                 const double dd = sums_finish<M>(s, c, p0 + lane, pa, a);
                 if (MODE == 4) dsum += dd;
             }
