@@ -363,7 +363,7 @@ void fill_solver_const(sphgpu_scene* h) {
 
 template <class T>
 int dalloc(sphgpu_scene* h, T** p, size_t n) {
-    cudaError_t e = cudaMalloc((void**)p, std::max<size_t>(n, 1) * sizeof(T));
+    cudaError_t e = dev_alloc(p, std::max<size_t>(n, 1) * sizeof(T));
     if (e != cudaSuccess) {
         h->err = std::string("cudaMalloc: ") + cudaGetErrorString(e);
         return SPHGPU_ENOMEM;
@@ -426,9 +426,9 @@ int alloc_scene(sphgpu_scene* h) {
     for (float4* c4 : {d.cA, d.cB, d.cC, d.cA_s, d.cB_s, d.cC_s, d.ap}) cudaMemsetAsync(c4, 0, sizeof(float4) * n, h->stream);
     // CUB scan scratch
     cub::DeviceScan::ExclusiveSum(nullptr, h->cub_bytes, d.cell_count, d.cell_start, h->g.nkeys + 1, h->stream);
-    if (cudaMalloc(&h->cub_tmp, h->cub_bytes + 16) != cudaSuccess) return SPHGPU_ENOMEM;
-    if (cudaMallocHost((void**)&h->h_stats, sizeof(DevStats)) != cudaSuccess) return SPHGPU_ENOMEM;
-    if (cudaMallocHost((void**)&h->h_cont, sizeof(int)) != cudaSuccess) return SPHGPU_ENOMEM;
+    if (dev_alloc(&h->cub_tmp, h->cub_bytes + 16) != cudaSuccess) return SPHGPU_ENOMEM;
+    if (host_alloc(&h->h_stats, sizeof(DevStats)) != cudaSuccess) return SPHGPU_ENOMEM;
+    if (host_alloc(&h->h_cont, sizeof(int)) != cudaSuccess) return SPHGPU_ENOMEM;
     memset(h->h_stats, 0, sizeof(DevStats));
     float dt = h->P.dt;
     cudaMemcpyAsync(d.dt, &dt, sizeof(float), cudaMemcpyHostToDevice, h->stream);
@@ -1264,8 +1264,8 @@ int rigid_reserve(sphgpu_scene* h, int n) {
     double* hout = nullptr;
     if (dalloc(h, &st, 25 * (size_t)cap) || dalloc(h, &out, 6 * (size_t)cap) || dalloc(h, &tk, cap))
         return SPHGPU_ENOMEM;
-    if (cudaMallocHost((void**)&hst, sizeof(float) * 25 * cap) != cudaSuccess ||
-        cudaMallocHost((void**)&hout, sizeof(double) * (6 * cap + 1)) != cudaSuccess)
+    if (host_alloc(&hst, sizeof(float) * 25 * cap) != cudaSuccess ||
+        host_alloc(&hout, sizeof(double) * (6 * cap + 1)) != cudaSuccess)
         return SPHGPU_ENOMEM;
     memset(hst, 0, sizeof(float) * 25 * cap);
     memset(hout, 0, sizeof(double) * (6 * cap + 1));
@@ -1403,8 +1403,8 @@ static int create_impl(const SphParams* p, int device, int max_fluid, int nscene
         // per-scene state: grids, then one block for the BatchDev arrays
         const size_t S = (size_t)nscenes;
         const size_t bytes = S * (sizeof(float) + 10 * sizeof(int) + 3 * sizeof(double)) + 256 + sizeof(int);
-        if (cudaMalloc((void**)&h->d_geom, S * sizeof(GridGeom)) != cudaSuccess ||
-            cudaMalloc(&h->d_batch, bytes) != cudaSuccess) {
+        if (dev_alloc(&h->d_geom, S * sizeof(GridGeom)) != cudaSuccess ||
+            dev_alloc(&h->d_batch, bytes) != cudaSuccess) {
             r = SPHGPU_ENOMEM;
         } else {
             copy_sync(h->d_geom, h->sgeom.data(), S * sizeof(GridGeom), cudaMemcpyHostToDevice);
@@ -1797,16 +1797,15 @@ int sphgpu_step_host(sphgpu_t h, int solver, const float* xyz, const float* vel,
         const size_t b3 = sizeof(float) * 3 * (size_t)h->cap;
         if (!h->h_diff) {
             // all four or none: a partial allocation is released again
-            if (cudaMalloc((void**)&h->in_xyz, b3) != cudaSuccess ||
-                cudaMalloc((void**)&h->in_vel, b3) != cudaSuccess ||
-                cudaMalloc((void**)&h->d_diff, sizeof(int)) != cudaSuccess ||
-                cudaMallocHost((void**)&h->h_diff, sizeof(int)) != cudaSuccess) {
+            if (dev_alloc(&h->in_xyz, b3) != cudaSuccess ||
+                dev_alloc(&h->in_vel, b3) != cudaSuccess ||
+                dev_alloc(&h->d_diff, sizeof(int)) != cudaSuccess ||
+                host_alloc(&h->h_diff, sizeof(int)) != cudaSuccess) {
                 for (void* q : {(void*)h->in_xyz, (void*)h->in_vel, (void*)h->d_diff})
                     if (q) cudaFree(q);
                 h->in_xyz = h->in_vel = nullptr;
                 h->d_diff = nullptr;
                 h->h_diff = nullptr;
-                cudaGetLastError();  // the failed allocation's error, reported here instead
                 h->err = "out of device memory (host-step input buffers)";
                 return SPHGPU_ENOMEM;
             }
@@ -2422,16 +2421,16 @@ int sphgpu_mlp_create(int device, int dataset_cap, uint64_t seed, sphgpu_mlp_t* 
     m->device = device;
     cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking);
     MlpDev& d = m->m;
-    bool ok = cudaMalloc(&d.master, sizeof(float) * MLP_NPARAM_PAD) == cudaSuccess &&
-              cudaMalloc(&d.grad, sizeof(float) * MLP_NPARAM_PAD) == cudaSuccess &&
-              cudaMalloc(&d.adam_m, sizeof(float) * MLP_NPARAM_PAD) == cudaSuccess &&
-              cudaMalloc(&d.adam_v, sizeof(float) * MLP_NPARAM_PAD) == cudaSuccess &&
-              cudaMalloc(&d.w_bf16, sizeof(__nv_bfloat16) * MLP_NPARAM_PAD) == cudaSuccess &&
-              cudaMalloc(&d.loss, sizeof(float)) == cudaSuccess &&
-              cudaMalloc(&d.norm, sizeof(float) * (2 * MLP_IN + 2)) == cudaSuccess &&
-              cudaMalloc(&m->ds_count, sizeof(int)) == cudaSuccess &&
-              cudaMalloc(&m->dsX, sizeof(float) * MLP_IN * ((size_t)dataset_cap + 1)) == cudaSuccess &&
-              cudaMalloc(&m->dsy, sizeof(float) * ((size_t)dataset_cap + 1)) == cudaSuccess;
+    bool ok = dev_alloc(&d.master, sizeof(float) * MLP_NPARAM_PAD) == cudaSuccess &&
+              dev_alloc(&d.grad, sizeof(float) * MLP_NPARAM_PAD) == cudaSuccess &&
+              dev_alloc(&d.adam_m, sizeof(float) * MLP_NPARAM_PAD) == cudaSuccess &&
+              dev_alloc(&d.adam_v, sizeof(float) * MLP_NPARAM_PAD) == cudaSuccess &&
+              dev_alloc(&d.w_bf16, sizeof(__nv_bfloat16) * MLP_NPARAM_PAD) == cudaSuccess &&
+              dev_alloc(&d.loss, sizeof(float)) == cudaSuccess &&
+              dev_alloc(&d.norm, sizeof(float) * (2 * MLP_IN + 2)) == cudaSuccess &&
+              dev_alloc(&m->ds_count, sizeof(int)) == cudaSuccess &&
+              dev_alloc(&m->dsX, sizeof(float) * MLP_IN * ((size_t)dataset_cap + 1)) == cudaSuccess &&
+              dev_alloc(&m->dsy, sizeof(float) * ((size_t)dataset_cap + 1)) == cudaSuccess;
     if (!ok) {
         sphgpu_mlp_destroy(m);
         return SPHGPU_ENOMEM;
@@ -2557,7 +2556,7 @@ static int mlp_ensure_gpart(sphgpu_mlp_t m, int rows) {
     if (m->m.gpart) cudaFree(m->m.gpart);
     m->m.gpart = nullptr;
     m->gpart_blocks = 0;
-    if (cudaMalloc(&m->m.gpart, sizeof(float) * ((size_t)blocks * MLP_NPARAM_PAD + blocks)) != cudaSuccess) {
+    if (dev_alloc(&m->m.gpart, sizeof(float) * ((size_t)blocks * MLP_NPARAM_PAD + blocks)) != cudaSuccess) {
         m->m.gpart = nullptr;
         m->err = "cudaMalloc failed (training gradient slots)";
         return SPHGPU_ENOMEM;
@@ -2616,8 +2615,8 @@ int sphgpu_mlp_gradient(sphgpu_mlp_t m, const float* X, const float* y, int n, f
     if (!m || !X || !y || n <= 0 || !grad) return SPHGPU_EINVAL;
     cudaSetDevice(m->device);
     float *dX = nullptr, *dy = nullptr;
-    if (cudaMalloc(&dX, sizeof(float) * MLP_IN * (size_t)n) != cudaSuccess ||
-        cudaMalloc(&dy, sizeof(float) * n) != cudaSuccess) {
+    if (dev_alloc(&dX, sizeof(float) * MLP_IN * (size_t)n) != cudaSuccess ||
+        dev_alloc(&dy, sizeof(float) * n) != cudaSuccess) {
         cudaFree(dX);
         return SPHGPU_ENOMEM;
     }
@@ -2648,8 +2647,8 @@ int sphgpu_mlp_predict(sphgpu_mlp_t m, const float* X, float* y, int n) {
     if (!n) return 0;
     cudaSetDevice(m->device);
     float *dX = nullptr, *dy = nullptr;
-    if (cudaMalloc(&dX, sizeof(float) * MLP_IN * (size_t)n) != cudaSuccess ||
-        cudaMalloc(&dy, sizeof(float) * n) != cudaSuccess) {
+    if (dev_alloc(&dX, sizeof(float) * MLP_IN * (size_t)n) != cudaSuccess ||
+        dev_alloc(&dy, sizeof(float) * n) != cudaSuccess) {
         cudaFree(dX);
         return SPHGPU_ENOMEM;
     }

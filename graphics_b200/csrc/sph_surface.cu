@@ -870,9 +870,8 @@ template <class T>
 int salloc(sphgpu_surface* s, T** p, size_t n) {
     if (*p) cudaFree(*p);
     *p = nullptr;
-    cudaError_t e = cudaMalloc((void**)p, std::max<size_t>(n, 1) * sizeof(T));
+    cudaError_t e = dev_alloc(p, std::max<size_t>(n, 1) * sizeof(T));
     if (e != cudaSuccess) {
-        cudaGetLastError();  // reported here, not by a later call's check
         s->err = std::string("cudaMalloc: ") + cudaGetErrorString(e);
         return SPHGPU_ENOMEM;
     }

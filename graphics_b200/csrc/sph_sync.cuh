@@ -1,4 +1,4 @@
-// sph_sync.cuh -- host-synchronous memory operations for the entry points.
+// sph_sync.cuh -- host-synchronous memory operations and allocations for the entry points.
 //
 // Every handle works on its own non-blocking streams, which are not ordered
 // with the legacy default stream that cudaMemcpy, cudaMemcpy2D and
@@ -26,4 +26,20 @@ inline cudaError_t copy2d_sync(void* dst, size_t dpitch, const void* src, size_t
 inline cudaError_t memset_sync(void* p, int value, size_t bytes) {
     const cudaError_t e = cudaMemset(p, value, bytes);
     return e == cudaSuccess ? cudaStreamSynchronize(cudaStreamLegacy) : e;
+}
+
+// Allocations whose failure the entry point reports itself (SPHGPU_ENOMEM): the
+// runtime keeps it as its last error too, which the next call that looks there,
+// on whatever handle, would take for its own.
+template <class T>
+inline cudaError_t dev_alloc(T** p, size_t bytes) {
+    const cudaError_t e = cudaMalloc((void**)p, bytes);
+    if (e != cudaSuccess) cudaGetLastError();
+    return e;
+}
+template <class T>
+inline cudaError_t host_alloc(T** p, size_t bytes) {
+    const cudaError_t e = cudaMallocHost((void**)p, bytes);
+    if (e != cudaSuccess) cudaGetLastError();
+    return e;
 }
