@@ -91,8 +91,8 @@ def test_more_than_2_31_triangles():
         sf = surface_field()
         sf.surface_setup([0.0] * 3, [0.01 * (n - 1) - 0.025] * 3, 0.01, 0.02, 0.01)
         assert [int(v) for v in sf.grid_num] == [n] * 3
-        i = np.arange(n)
-        f = ((i[:, None, None] + i[None, :, None] + i[None, None, :]) & 1).astype(np.float32)
+        i = (np.arange(n) & 1).astype(np.uint8)
+        f = (i[:, None, None] ^ i[None, :, None] ^ i[None, None, :]).astype(np.float32)
         sf.set_field(f)
         head = np.zeros((8, 3, 3), np.float32)
         total = sf.lib.sphgpu_surface_mesh(sf.h, 0.5, 0, head.ctypes.data_as(C.POINTER(C.c_float)), len(head))
