@@ -1488,7 +1488,9 @@ int sphgpu_set_params(sphgpu_t h, const SphParams* p) {
     return 0;
 }
 
-// Boundary particles of all scenes (scene == NULL: the single scene).
+// Boundary particles of all scenes (scene == NULL: the single scene).  The walls
+// that are there stay until the new ones are known to be inside the grid and
+// their arrays are allocated: an error leaves the handle as it was.
 static int set_boundary_impl(sphgpu_t h, int n, const float* xyz, const int* solid_id, const int* scene, const float* volume) {
     if (!h || n < 0 || (n > 0 && !xyz)) return SPHGPU_EINVAL;
     cudaSetDevice(h->device);
@@ -1496,19 +1498,19 @@ static int set_boundary_impl(sphgpu_t h, int n, const float* xyz, const int* sol
     if (scene)
         for (int i = 0; i < n; ++i)
             if (scene[i] < 0 || scene[i] >= h->nscenes) { h->err = "boundary scene index out of range"; return SPHGPU_EINVAL; }
-    free_rigid(h);
-    if (d.bpos) { cudaFree(d.bpos); cudaFree(d.bvel); cudaFree(d.bgid); cudaFree(d.bpv); d.bpos = nullptr; }
-    for (void* q : {(void*)d.bsid, (void*)d.bnbr, (void*)d.bncount, (void*)d.bivs, (void*)d.bivo})
-        if (q) cudaFree(q);
-    d.bsid = d.bnbr = d.bncount = nullptr;
-    d.bivs = d.bivo = nullptr;
-    h->nb = n;
-    d.nb = n;
     std::vector<float4> bp(n);
     for (int i = 0; i < n; ++i) bp[i] = make_float4(xyz[3 * i], xyz[3 * i + 1], xyz[3 * i + 2], volume ? volume[i] : 0.f);
-    if (dalloc(h, &d.bpos, n) || dalloc(h, &d.bvel, n) || dalloc(h, &d.bgid, n) || dalloc(h, &d.bpv, 2 * (size_t)n))
+    struct Walls {
+        float4 *bpos = nullptr, *bvel = nullptr, *bpv = nullptr;
+        int *bgid = nullptr, *keys = nullptr;
+        ~Walls() {
+            for (void* q : {(void*)bpos, (void*)bvel, (void*)bpv, (void*)bgid, (void*)keys})
+                if (q) cudaFree(q);
+        }
+    } w;
+    if (dalloc(h, &w.bpos, n) || dalloc(h, &w.bvel, n) || dalloc(h, &w.bgid, n) || dalloc(h, &w.bpv, 2 * (size_t)n) ||
+        dalloc(h, &w.keys, n))
         return SPHGPU_ENOMEM;
-    d.bpf = d.bpv;
     // cell keys on the device, each particle with its scene's grid
     std::vector<int> keys(n);
     {
@@ -1517,21 +1519,18 @@ static int set_boundary_impl(sphgpu_t h, int n, const float* xyz, const int* sol
         if (scene) std::stable_sort(ord.begin(), ord.end(), [&](int a, int b) { return scene[a] < scene[b]; });
         std::vector<float4> tmp(n);
         for (int i = 0; i < n; ++i) tmp[i] = bp[ord[i]];
-        int* dkeys = nullptr;
-        if (dalloc(h, &dkeys, n)) return SPHGPU_ENOMEM;
-        CK(copy_sync(d.bpos, tmp.data(), sizeof(float4) * n, cudaMemcpyHostToDevice));
+        CK(copy_sync(w.bpos, tmp.data(), sizeof(float4) * n, cudaMemcpyHostToDevice));
         for (int a = 0; a < n;) {
             int b = a;
             const int sc = scene ? scene[ord[a]] : 0;
             while (b < n && (scene ? scene[ord[b]] : 0) == sc) ++b;
             const GridGeom& G = h->nscenes > 1 ? h->sgeom[sc] : h->g;
-            launch_boundary_keys(d.bpos + a, b - a, G, dkeys + a, h->stream);
+            launch_boundary_keys(w.bpos + a, b - a, G, w.keys + a, h->stream);
             a = b;
         }
         CK(cudaStreamSynchronize(h->stream));
         std::vector<int> k2(n);
-        CK(copy_sync(k2.data(), dkeys, sizeof(int) * n, cudaMemcpyDeviceToHost));
-        cudaFree(dkeys);
+        CK(copy_sync(k2.data(), w.keys, sizeof(int) * n, cudaMemcpyDeviceToHost));
         for (int i = 0; i < n; ++i) keys[ord[i]] = k2[i];
     }
     // reference insertion rank: solids in order, each in index order (the
@@ -1552,6 +1551,19 @@ static int set_boundary_impl(sphgpu_t h, int n, const float* xyz, const int* sol
             h->err = "boundary particle outside the grid";
             return SPHGPU_EINVAL;
         }
+    free_rigid(h);
+    for (void* q : {(void*)d.bsid, (void*)d.bnbr, (void*)d.bncount, (void*)d.bivs, (void*)d.bivo})
+        if (q) cudaFree(q);
+    d.bsid = d.bnbr = d.bncount = nullptr;
+    d.bivs = d.bivo = nullptr;
+    // the old arrays go with w
+    std::swap(d.bpos, w.bpos);
+    std::swap(d.bvel, w.bvel);
+    std::swap(d.bgid, w.bgid);
+    std::swap(d.bpv, w.bpv);
+    d.bpf = d.bpv;
+    h->nb = n;
+    d.nb = n;
     std::vector<int> perm(n);
     std::iota(perm.begin(), perm.end(), 0);
     std::sort(perm.begin(), perm.end(), [&](int a, int b) {

@@ -1,4 +1,4 @@
-"""Handles after a call that found no device memory (GPU)."""
+"""Handles after a call that failed, for want of memory or on its input (GPU)."""
 import numpy as np
 import pytest
 
@@ -24,6 +24,27 @@ def test_a_failed_handle_does_not_fail_others():
         g.step("dfsph", 2)
         g.stage("neighbourSearch")
         out.append((g.get("position"), g.get("density")))
+        g.close()
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("solver", ["dfsph", "wcsph", "pcisph", "iisph"])
+def test_refused_walls_leave_the_ones_that_are_there(solver):
+    """Fewer walls than before, one of them outside the grid: an error, and the
+    scene goes on with its own."""
+    sc = small_dam_break((9, 8, 7), r=0.025, seed=2)
+    out = []
+    for attempt in (False, True):
+        g = scene_to_gpu(sc, dt=5e-4, nu=1e-3, soundSpeed_cs=20.0)
+        g.step(solver, 1)
+        if attempt:
+            few = np.array([[0.01, 0.01, 0.01], [100.0, 0.0, 0.0], [0.02, 0.01, 0.01]], np.float32)
+            with pytest.raises(SphGpuError) as e:
+                g.set_boundary(few)
+            assert e.value.code == _lib.EINVAL
+        g.step(solver, 2)
+        out.append((g.get("position"), g.get("density"), g.get_boundary("position"), g.get_boundary("volume")))
         g.close()
     for a, b in zip(*out):
         np.testing.assert_array_equal(a, b)
